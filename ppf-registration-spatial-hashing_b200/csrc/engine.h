@@ -21,13 +21,16 @@ constexpr int kBins = 31;
 // Vote kernel launch shape: one 1024-thread block per SM.
 constexpr int kVoteThreads = 1024;
 constexpr int kVoteWarps = kVoteThreads / 32;
-// Shared memory of the vote block besides its accumulator: per scene pair of
-// a tile its sub-run start and length, angle word, frame vector (y, z) and
-// segment offset (+1 entry).
-constexpr int kVoteQueueBytes = kVoteThreads * (4 + 4 + 4 + 8) + (kVoteThreads + 4) * 4;
-// Accumulator words of a chunk: one 32-bit counter per (m_r, alpha bin) cell
-// (the reference counts votes in unsigned int too, include/impl/util.hpp:30-52).
-inline size_t vote_acc_words(uint32_t chunk) { return ((size_t)chunk * kBins + 3) & ~size_t(3); }
+// Most m_r rows of a chunk: m_r mod chunk takes the 11 bits above an entry's
+// 21-bit angle, and ppf_model_num_chunks reports the chunks.  (1659 rows of
+// 31 32-bit counters were what one block's shared memory held; at 64 bytes a
+// row they now share it with the scene pairs of one reference point.)
+constexpr uint32_t kMaxChunk = 1659;
+// Feature table of a model (ModelTables::lut): distance rows with a run per
+// angle combination, and rows whose flag says whether any key of theirs
+// belongs to the model.
+constexpr uint32_t kLutRows = 128;
+constexpr uint32_t kFlagRows = 1024;
 // Angle quantum on the host (include/kernel.h:16 evaluated in float).
 #define PPF_D_ANGLE_HOST ((2.0f * 3.141592654f) / float(30))
 
@@ -48,12 +51,8 @@ struct Context {
   // (points, d_dist, threshold) emitted; sizes the next batch's buffers when
   // the same model is built again
   std::unordered_map<uint64_t, size_t> cand_hints;
-  // vote segment length chosen by the tuner per model signature
-  // (tune_vote_segments); PPF_B200_TUNE=0 keeps the default
-  std::unordered_map<uint64_t, uint32_t> seg_tuned;
-  bool tune = true;
   uint32_t forced_seg_shift = 0;  // PPF_B200_VOTE_SEGMENT=<2^k>: every model uses it
-  DevBuf tune_counters;
+  DevBuf vote_spill;  // per vote block: 32-bit counters of one chunk (reserve_vote_spill)
   size_t cand_cap = size_t(1) << 24;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   int vote_smem_limit = 0;  // max dynamic shared memory per vote block
@@ -77,16 +76,26 @@ struct ModelTables {
   size_t P = 0;
   DevBuf keys;           // uint32 sorted keys
   DevBuf pairs;          // uint32 pair index r*n + i (the hash array's data map)
-  DevBuf entries;        // uint32 (m_r mod chunk) << 21 | 21-bit angle of u,
-                         // vote order: by key, then m_r, then a hash of the pair
+  // Vote order: by run, then chunk of m_r, then buckets of 2^r_shift of
+  // R = 30 x angle mod 2^21 (the angle's position inside an alpha bin), each
+  // block of 128 dealt to lanes by m_r mod 32
+  DevBuf entries;        // uint32 (m_r mod chunk) << 21 | 21-bit angle of u
   DevBuf epairs;         // uint32 pair index of each entry (vote order)
+  uint32_t r_shift = 0;
   // runs
   size_t K = 0;
   DevBuf uniq, first, count;  // uint32 each
+  DevBuf run_maxl;            // uint32: most entries of the run that share one m_r
   DevBuf run_flags;           // uint8: 1 = run holds a degenerate pair (exact bins only)
   // key -> run open-addressing table (key 0 is the empty marker)
   DevBuf ht_keys, ht_runs;
   uint32_t ht_mask = 0;
+  // Runs of quantised features, for scenes with the model's own quantum:
+  // lut[nd * 4913 + angles] for nd < kLutRows (pair_angles; 0xffffffff: none),
+  // row_flags bit nd set if any feature of distance index nd < kFlagRows has a
+  // run.  lut_quantum: the quantum they hold for (0: no table)
+  DevBuf lut, row_flags;
+  float lut_quantum = 0;
   // m_r chunking of the vote accumulator
   uint32_t chunk = 0, n_chunks = 0;
   DevBuf split;  // uint32 [K * (n_chunks + 1)] first run position per chunk
@@ -130,10 +139,6 @@ struct Model {
   float vote_count_threshold = 0.4f;
   bool cpu_clustering = false, use_l1_norm = false, use_averaged_clusters = false;
   size_t cand_hint = 0;  // candidate cells of the last vote pass (sizes batch buffers)
-  // log2 of the vote pass's segment length (entries a warp streams per
-  // segment); 0 until the tuner has chosen it (the default is used)
-  // (atomic: the workers of a server may tune one library model at once)
-  std::atomic<uint32_t> seg_shift{0};
   LookupState last;
 };
 
@@ -163,6 +168,9 @@ struct VoteResult {
 // Runs the vote pass.  emit_all: emit every nonzero cell (no threshold);
 // floor >= 0 forces the emission floor.  Candidates land in
 // ctx.cand_codes / ctx.cand_counts.
+void init_vote_kernels(int smem_limit);
+// The vote blocks' 32-bit counters (ctx.vote_spill).
+void reserve_vote_spill(Context& ctx);
 VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit_all, float floor);
 // One request of a batched vote pass: its candidate cells land in its own
 // buffers (cap cells, grown if they do not fit).
@@ -184,12 +192,16 @@ void vote_cells_noalloc(Context& ctx, const Model& m, const float* xyz, const fl
                         uint64_t n, uint32_t ref_df, float vote_floor, uint64_t* codes,
                         uint32_t* counts, uint64_t capacity, uint64_t* n_out, uint32_t* max_out);
 
-// Default log2 segment length of the vote pass and the tuner's candidates.
+// log2 of the vote pass's segment length: 4096 entries unless
+// PPF_B200_VOTE_SEGMENT says otherwise.  A unit of the vote phase is a quarter
+// of it and shrinks where units are few, so the length hardly matters any
+// more (2048 / 4096 / 8192: 5.99 / 5.87 / 5.86 ms for a 2000-point model's
+// vote pass); it used to be timed per model on the first lookup, which cost
+// up to three lookups' worth of launches.
 constexpr uint32_t kSegShiftDefault = 12;
-// Chooses the vote pass's segment length for model m on its first lookup
-// (per model signature, cached in the context): short vote launches over a
-// sample of the work items of (m, s), counting only, one per candidate.
-void tune_vote_segments(Context& ctx, Model& m, const SceneData& s, uint64_t signature);
+inline uint32_t vote_segment_shift(const Context& ctx) {
+  return ctx.forced_seg_shift ? ctx.forced_seg_shift : kSegShiftDefault;
+}
 uint64_t model_signature(const Model& m);
 
 // ---- poses and clustering (pose.cu)

@@ -55,51 +55,147 @@ __global__ void pair_keys_kernel(const float4* __restrict__ pts, const float4* _
   }
 }
 
-// Vote order of the run entries: by key, then m_r, then a hash of the pair
-// index.  Grouping a run by m_r lets the vote pass split it into m_r chunks;
-// the hash scatters the pairs of one m_r over angles, so that neighbouring
-// lanes of a warp rarely count into the same (m_r, bin) cell even when the
-// cloud's points come in scan order.
-__global__ void order_words_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pairs,
-                                   size_t P, uint32_t n, unsigned long long* __restrict__ words) {
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < P;
-       j += (size_t)gridDim.x * blockDim.x) {
-    uint32_t pr = pairs[j];
-    uint32_t mr = pr / n;
-    words[j] = ((unsigned long long)keys[j] << 32) | (mr << 16) | ((pr * 0x9E3779B1u) >> 16);
+// Angle word of model pair pr: (m_r mod chunk) << 21 | angle21(u), u = the
+// pair's second point in the frame of the first.  A u that is (numerically)
+// zero cannot be binned from angles; its run is flagged for exact binning.
+__device__ __forceinline__ uint32_t pair_entry(uint32_t pr, uint32_t n, uint32_t chunk, const float4* __restrict__ pts,
+                                               const float4* __restrict__ r1, const float4* __restrict__ r2,
+                                               bool& degenerate) {
+  const uint32_t mr = pr / n, mi = pr - mr * n;
+  FrameYZ f;
+  f.r1 = r1[mr];
+  f.r2 = r2[mr];
+  const float4 q4 = pts[mi];
+  const float2 u = frame_point_yz(f, make_float3(q4.x, q4.y, q4.z));
+  degenerate = fabsf(u.x) + fabsf(u.y) < 1e-12f || !isfinite(u.x) || !isfinite(u.y);
+  return ((mr % chunk) << PPF_ANGLE_BITS) | angle21(u);
+}
+
+// Sort word of each pair for the vote order: run, chunk of m_r, then the top
+// r_bits of R = 30 x angle mod 2^21.  Also the run's exact flag and the most
+// pairs of the run that share one m_r (the pairs of a run come in m_r order).
+// The runs of 32 consecutive pairs follow from one search and a ballot.
+template <typename W>
+__global__ void order_words_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pairs, size_t P,
+                                   uint32_t n, uint32_t chunk, const float4* __restrict__ pts,
+                                   const float4* __restrict__ r1, const float4* __restrict__ r2,
+                                   const uint32_t* __restrict__ first, size_t K, int chunk_bits, int r_bits,
+                                   W* __restrict__ words, uint8_t* __restrict__ run_flags,
+                                   uint32_t* __restrict__ run_maxl) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (size_t j0 = blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31u); j0 < P;
+       j0 += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = j0 + lane;
+    const bool in = j < P;
+    size_t lo = 0, hi = K;  // run of j0: last run start <= j0
+    while (hi - lo > 1) {
+      const size_t mid = (lo + hi) >> 1;
+      if (first[mid] <= j0) lo = mid;
+      else hi = mid;
+    }
+    const uint32_t key = in ? keys[j] : 0u;
+    const bool head = in && (j == 0 || keys[j - 1] != key);
+    const uint32_t heads = __ballot_sync(0xffffffffu, head) & ~1u;  // starts after j0
+    if (!in) continue;
+    const size_t run = lo + __popc(heads & (0xffffffffu >> (31u - lane)));
+    const uint32_t pr = pairs[j], mr = pr / n;
+    bool degenerate;
+    const uint32_t e = pair_entry(pr, n, chunk, pts, r1, r2, degenerate);
+    if (degenerate) run_flags[run] = 1;
+    const uint32_t r = ((e & ((1u << PPF_ANGLE_BITS) - 1u)) * PPF_N_ANGLE) & ((1u << PPF_ANGLE_BITS) - 1u);
+    words[j] = (((W)run << chunk_bits | (W)(mr / chunk)) << r_bits) | (W)(r >> (PPF_ANGLE_BITS - r_bits));
+    // lengths of the (run, m_r) groups that start here: up to the next start,
+    // or, for the warp's last group, counted 32 pairs at a time beyond it
+    const bool start = head || j == 0 || pairs[j - 1] / n != mr;
+    const uint32_t lanes = P - j0 >= 32 ? 0xffffffffu : (1u << (P - j0)) - 1u;
+    const uint32_t starts = __ballot_sync(lanes, start);
+    if (!starts) continue;
+    const int last = 31 - __clz(starts);
+    const uint32_t last_key = __shfl_sync(lanes, key, last), last_mr = __shfl_sync(lanes, mr, last);
+    uint32_t tail = __popc(lanes) - last;
+    for (size_t b = j0 + 32;; b += 32) {
+      const bool same = b + lane < P && keys[b + lane] == last_key && pairs[b + lane] / n == last_mr;
+      const uint32_t other = ~__ballot_sync(lanes, same) & lanes;
+      tail += other ? __ffs(other) - 1 : 32;
+      if (other) break;
+    }
+    if (start) {
+      const uint32_t later = starts & ~(0xffffffffu >> (31u - lane));
+      const uint32_t l = later ? __ffs(later) - 1 - lane : tail;
+      if (l > run_maxl[run]) atomicMax(run_maxl + run, l);
+    }
   }
 }
 
-// Vote entry of each pair in vote order: (m_r mod chunk) << 21 | angle21(u),
-// u = the pair's second point in the frame of the first: the top 11 bits are
-// the pair's m_r inside its chunk, so the vote kernel forms the cell index
-// row * 31 + bin with one multiply-add.  A pair whose u is
-// (numerically) zero cannot be binned from angles; its run is flagged for
-// exact binning.
-__global__ void entries_kernel(const uint32_t* __restrict__ epairs, size_t P, uint32_t n,
-                               uint32_t chunk, const float4* __restrict__ pts, const float4* __restrict__ r1,
-                               const float4* __restrict__ r2, const uint32_t* __restrict__ first,
-                               size_t K, uint32_t* __restrict__ entries,
-                               uint8_t* __restrict__ run_flags) {
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < P;
-       j += (size_t)gridDim.x * blockDim.x) {
-    uint32_t pr = epairs[j];
-    uint32_t mr = pr / n, mi = pr - mr * n;
-    FrameYZ f;
-    f.r1 = r1[mr];
-    f.r2 = r2[mr];
-    float4 q4 = pts[mi];
-    float2 u = frame_point_yz(f, make_float3(q4.x, q4.y, q4.z));
-    entries[j] = ((mr % chunk) << PPF_ANGLE_BITS) | angle21(u);
-    if (fabsf(u.x) + fabsf(u.y) < 1e-12f || !isfinite(u.x) || !isfinite(u.y)) {
-      // run of position j: last run start <= j
-      size_t lo = 0, hi = K;
-      while (hi - lo > 1) {
-        size_t mid = (lo + hi) >> 1;
-        if (first[mid] <= j) lo = mid;
-        else hi = mid;
+// Vote entries of each sub-run (run, chunk), from the sorted pairs.  The warp
+// that takes a whole block of 128 adds 32 of its entries at a time to rows
+// m_r of the vote pass's accumulator, in bank m_r mod 32.  The block is
+// ordered by m_r mod 32 and dealt round to four such passes, so that a value
+// with n entries costs at most ceil(n / 4) accesses a pass: 8.9 accesses a
+// block on average where the order of R gives 14.1 and no order less than the
+// most frequent value's 8.6 (random values).  A warp per sub-run and
+// blockIdx.y; it reads and writes only its own blocks.
+constexpr int kEntryBlock = 128;
+__global__ void entries_kernel(uint32_t* __restrict__ epairs, uint32_t n, uint32_t chunk,
+                               const float4* __restrict__ pts, const float4* __restrict__ r1,
+                               const float4* __restrict__ r2, const uint32_t* __restrict__ split, size_t K,
+                               uint32_t n_chunks, uint32_t* __restrict__ entries) {
+  const uint32_t lane = threadIdx.x & 31;
+  const size_t n_sub = K * n_chunks;
+  for (size_t s = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5; s < n_sub;
+       s += ((size_t)gridDim.x * blockDim.x) >> 5) {
+    const size_t run = s / n_chunks;
+    const uint32_t* sp = split + run * (n_chunks + 1) + (s - run * n_chunks);
+    const size_t lo = sp[0], hi = sp[1];
+    for (size_t b = lo + (size_t)blockIdx.y * kEntryBlock; b < hi; b += (size_t)gridDim.y * kEntryBlock) {
+      uint32_t pr[4], e[4], at[4];
+      const bool whole = b + kEntryBlock <= hi;
+      bool degenerate;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        at[k] = 32u * k + lane;
+        pr[k] = b + at[k] < hi ? epairs[b + at[k]] : 0u;
+        e[k] = pair_entry(pr[k], n, chunk, pts, r1, r2, degenerate);
       }
-      run_flags[lo] = 1;
+      if (whole) {
+        // counting sort by m_r mod 32: lane v holds the number of entries with
+        // value v
+        uint32_t have = 0, rank[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t v = (e[k] >> PPF_ANGLE_BITS) & 31u;
+          const uint32_t peers = __match_any_sync(0xffffffffu, v);
+          rank[k] = __shfl_sync(0xffffffffu, have, v) + __popc(peers & ((1u << lane) - 1u));
+          uint32_t same = 0xffffffffu;  // lanes whose value is this lane's index
+#pragma unroll
+          for (int bit = 0; bit < 5; ++bit) {
+            const uint32_t set = __ballot_sync(0xffffffffu, (v >> bit) & 1u);
+            same &= (lane >> bit) & 1u ? set : ~set;
+          }
+          have += __popc(same);
+        }
+        uint32_t below = have;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, below, o);
+          if (lane >= (uint32_t)o) below += y;
+        }
+        below -= have;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t r = __shfl_sync(0xffffffffu, below, (e[k] >> PPF_ANGLE_BITS) & 31u) + rank[k];
+          at[k] = 32u * (r & 3u) + (r >> 2);
+        }
+      }
+      __syncwarp();  // the block is read before it is rewritten
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (b + at[k] < hi) {
+          entries[b + at[k]] = e[k];
+          epairs[b + at[k]] = pr[k];
+        }
+      }
+      __syncwarp();
     }
   }
 }
@@ -126,8 +222,36 @@ __global__ void ht_build_kernel(const uint32_t* __restrict__ uniq, size_t K, uin
   }
 }
 
+// The feature table (ModelTables::lut): a block per distance index nd, every
+// combination of three angle indices looked up by its key.  Exact, collisions
+// of the 32-bit keys included, so a scene pair need not be hashed, and pairs
+// whose row has no run (most pairs of a large scene are further apart than
+// any model pair) need no angles at all.
+__global__ void __launch_bounds__(256) lut_kernel(const uint32_t* __restrict__ ht_keys,
+                                                  const uint32_t* __restrict__ ht_runs, uint32_t mask, float d_dist,
+                                                  uint32_t* __restrict__ lut, uint32_t* __restrict__ row_flags) {
+  const uint32_t nd = blockIdx.x;
+  const uint32_t h1 = fnv1a_word(PPF_FNV_BASIS, __float_as_uint(__fmul_rn((float)nd, d_dist)));
+  bool any = false;
+  for (uint32_t c = threadIdx.x; c < kAngleCombos; c += blockDim.x) {
+    const uint32_t y = c / (kAngleValues * kAngleValues), z = c / kAngleValues % kAngleValues, w = c % kAngleValues;
+    const uint32_t key = fnv1a_word(fnv1a_word(fnv1a_word(h1, angle_word(y)), angle_word(z)), angle_word(w));
+    uint32_t run = 0xffffffffu;
+    uint32_t s = ht_slot(key, mask);
+    for (uint32_t probe = 0; key != 0u && probe <= mask; ++probe) {
+      const uint32_t k = ht_keys[s];
+      if (k == key) run = ht_runs[s];
+      if (k == key || k == 0u) break;
+      s = (s + 1) & mask;
+    }
+    if (nd < kLutRows) lut[nd * kAngleCombos + c] = run;
+    any = any || run != 0xffffffffu;
+  }
+  if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(row_flags + nd / 32, 1u << (nd % 32));
+}
+
 // split[r*(C+1) + c] = first position of run r whose m_r >= c*chunk
-// (entries of a run are in m_r order).
+// (entries of a run are in chunk order).
 __global__ void split_kernel(const uint32_t* __restrict__ epairs, uint32_t n,
                              const uint32_t* __restrict__ first,
                              const uint32_t* __restrict__ count, size_t K, uint32_t chunk,
@@ -294,45 +418,67 @@ void build_model(Context& ctx, ModelTables& t, const float* xyz, const float* nx
   // run tables (the hash array's unique keys, counts and first offsets)
   t.K = build_runs(t.keys.as<uint32_t>(), t.P, t.uniq, t.first, t.count, ctx.scratch, st, &ctx.launches);
 
-  // m_r chunks sized to the vote kernel's shared-memory accumulator
-  uint32_t max_chunk = 64;
-  // (m_r mod chunk fits the 11 bits above an entry's 21-bit angle)
-  while (vote_acc_words(max_chunk + 1) * 4 + kVoteQueueBytes <= (size_t)ctx.vote_smem_limit &&
-         max_chunk < (1u << (32 - PPF_ANGLE_BITS)))
-    ++max_chunk;
-  t.n_chunks = (t.n + max_chunk - 1) / max_chunk;
+  // m_r chunks: an accumulator of the vote kernel's shared memory each
+  t.n_chunks = (t.n + kMaxChunk - 1) / kMaxChunk;
   t.chunk = (t.n + t.n_chunks - 1) / t.n_chunks;
 
   // vote entries in vote order; epairs keeps each entry's pair index
   t.entries.reserve(t.P * sizeof(uint32_t));
   t.epairs.reserve(t.P * sizeof(uint32_t));
   t.run_flags.reserve(t.K);
+  t.run_maxl.reserve(t.K * sizeof(uint32_t));
   t.split.reserve(t.K * (t.n_chunks + 1) * sizeof(uint32_t));
   PPF_CUDA(cudaMemsetAsync(t.run_flags.ptr, 0, t.K, st));
+  PPF_CUDA(cudaMemsetAsync(t.run_maxl.ptr, 0, t.K * sizeof(uint32_t), st));
   {
-    DevBuf words;
-    words.reserve(t.P * sizeof(unsigned long long));
-    order_words_kernel<<<grid_for(t.P, 256), 256, 0, st>>>(t.keys.as<uint32_t>(), t.pairs.as<uint32_t>(),
-                                                            t.P, t.n, words.as<unsigned long long>());
+    auto bits_for = [](uint64_t x) {
+      int b = 0;
+      while (b < 64 && (x >> b) != 0) ++b;
+      return b;
+    };
+    // Sort word: run and chunk in as many bits as they need, and R in what is
+    // left of the next whole digit, at least 9 bits (512 buckets over an
+    // alpha bin; a block of 128 entries spans more than one of them unless
+    // its sub-run has over 65536 entries).  24 bits for the bench's first
+    // model, 32 for a 40000-point one: 3 or 4 passes over 8-byte elements.
+    const int run_bits = bits_for(t.K - 1), chunk_bits = bits_for(t.n_chunks - 1);
+    const int word_bits = (run_bits + chunk_bits + 9 + 7) / 8 * 8;
+    const int r_bits = std::min(word_bits - run_bits - chunk_bits, PPF_ANGLE_BITS);
+    t.r_shift = PPF_ANGLE_BITS - r_bits;
     PPF_CUDA(cudaMemcpyAsync(t.epairs.ptr, t.pairs.ptr, t.P * 4, cudaMemcpyDeviceToDevice, st));
-    PPF_CUDA(cudaGetLastError());
-    size_t l1 = ctx.sort64.launches();
-    ctx.sort64.sort(words.as<unsigned long long>(), t.epairs.as<uint32_t>(), false, t.P, 0, 64, st,
-                    ctx.flags.as<uint32_t>());
-    ctx.launches += ctx.sort64.launches() - l1 + 1;
+    auto order = [&](auto& sorter, auto* words) {
+      order_words_kernel<<<grid_for(t.P, 256), 256, 0, st>>>(
+          t.keys.as<uint32_t>(), t.pairs.as<uint32_t>(), t.P, t.n, t.chunk, t.pts.as<float4>(),
+          t.frame_r1.as<float4>(), t.frame_r2.as<float4>(), t.first.as<uint32_t>(), t.K, chunk_bits, r_bits, words,
+          t.run_flags.as<uint8_t>(), t.run_maxl.as<uint32_t>());
+      PPF_CUDA(cudaGetLastError());
+      const size_t l1 = sorter.launches();
+      sorter.sort(words, t.epairs.as<uint32_t>(), false, t.P, 0, run_bits + chunk_bits + r_bits, st,
+                  ctx.flags.as<uint32_t>());
+      ctx.launches += sorter.launches() - l1 + 1;
+    };
+    // (the words borrow the entries' buffer when they are 32-bit)
+    if (word_bits <= 32) {
+      order(ctx.sort32, t.entries.as<uint32_t>());
+    } else {
+      DevBuf words;
+      words.reserve(t.P * sizeof(unsigned long long));
+      order(ctx.sort64, words.as<unsigned long long>());
+    }
     // chunk boundaries of every run (entries are in chunk order within a run)
     split_kernel<<<grid_for(t.K, 256), 256, 0, st>>>(t.epairs.as<uint32_t>(), t.n, t.first.as<uint32_t>(),
                                                       t.count.as<uint32_t>(), t.K, t.chunk, t.n_chunks,
                                                       t.split.as<uint32_t>());
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
-    entries_kernel<<<grid_for(t.P, 256), 256, 0, st>>>(
-        t.epairs.as<uint32_t>(), t.P, t.n, t.chunk, t.pts.as<float4>(), t.frame_r1.as<float4>(),
-        t.frame_r2.as<float4>(), t.first.as<uint32_t>(), t.K, t.entries.as<uint32_t>(),
-        t.run_flags.as<uint8_t>());
+    const dim3 grid(grid_for(t.K * t.n_chunks, 8, 16), 8);
+    entries_kernel<<<grid, 256, 0, st>>>(t.epairs.as<uint32_t>(), t.n, t.chunk, t.pts.as<float4>(),
+                                         t.frame_r1.as<float4>(), t.frame_r2.as<float4>(), t.split.as<uint32_t>(),
+                                         t.K, t.n_chunks, t.entries.as<uint32_t>());
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
   }
+  reserve_vote_spill(ctx);
 
   // key -> run table, load factor <= 0.5
   uint32_t cap = 1024;
@@ -347,6 +493,16 @@ void build_model(Context& ctx, ModelTables& t, const float* xyz, const float* nx
   PPF_CUDA(cudaGetLastError());
 
   ctx.launches += 1;
+  if (d_dist >= kQuantMin) {
+    t.lut.reserve((size_t)kLutRows * kAngleCombos * sizeof(uint32_t));
+    t.row_flags.reserve(kFlagRows / 8);
+    PPF_CUDA(cudaMemsetAsync(t.row_flags.ptr, 0, kFlagRows / 8, st));
+    lut_kernel<<<kFlagRows, 256, 0, st>>>(t.ht_keys.as<uint32_t>(), t.ht_runs.as<uint32_t>(), t.ht_mask, d_dist,
+                                          t.lut.as<uint32_t>(), t.row_flags.as<uint32_t>());
+    PPF_CUDA(cudaGetLastError());
+    ctx.launches += 1;
+    t.lut_quantum = d_dist;
+  }
   unsigned long long* bad = reinterpret_cast<unsigned long long*>(ctx.flags.as<uint32_t>() + 8);
   if (ctx.checks) {
     PPF_CUDA(cudaMemsetAsync(bad, 0, 24, st));

@@ -84,6 +84,20 @@ __device__ __forceinline__ float norm4(float4 a) { return sqrtf(dot4(a, a)); }
 // x rounded down to a multiple of y, as x - fmodf(x, y) (src/cuda/kernel.cu:90-92).
 __device__ __forceinline__ float quant_down(float x, float y) { return x - fmodf(x, y); }
 
+// trunc(x / y) of non-negative x: the n for which quant_down(x, y) is
+// fl(n y).  fmodf is exact, so x - fmodf(x, y) rounds the real number n y, as
+// n * y does.  n comes from a multiplication by 1 / y, off by at most one
+// below 2^20, and the exact sign of one fma on either side.  Valid for y at
+// least kQuantMin (below it a remainder may be subnormal and flushed) and
+// x < 2^20 y.
+constexpr float kQuantMin = 1e-25f;
+__device__ __forceinline__ int quant_index(float x, float y, float inv_y) {
+  int n = (int)(x * inv_y);
+  if (__fmaf_rn(-(float)n, y, x) < 0.f) --n;
+  if (__fmaf_rn(-(float)(n + 1), y, x) >= 0.f) ++n;
+  return n;
+}
+
 // Point pair feature (|d|, angle(n1,d), angle(n2,d), angle(n1,n2))
 // (src/cuda/kernel.cu:109-122), then discretised (src/cuda/kernel.cu:94-100).
 __device__ __forceinline__ float4 pair_feature(float3 p1, float3 n1, float3 p2, float3 n2,
@@ -102,6 +116,29 @@ __device__ __forceinline__ float4 pair_feature(float3 p1, float3 n1, float3 p2, 
   f.z = quant_down(f.z, PPF_D_ANGLE);
   f.w = quant_down(f.w, PPF_D_ANGLE);
   return f;
+}
+
+// Quantised features as small integers: distance index nd (of quant_index)
+// and three angle indices of 0..15, or kAngleNaN for a NaN angle.  Their key
+// is feature_key of the floats they stand for (a NaN that went through an
+// addition has the one pattern 0x7fffffff).
+constexpr uint32_t kAngleValues = 17, kAngleNaN = 16;
+constexpr uint32_t kAngleCombos = kAngleValues * kAngleValues * kAngleValues;
+
+__device__ __forceinline__ uint32_t angle_word(uint32_t n) {
+  return n == kAngleNaN ? 0x7fffffffu : __float_as_uint(__fmul_rn((float)n, PPF_D_ANGLE));
+}
+
+__device__ __forceinline__ uint32_t angle_index(float angle) {
+  return isnan(angle) ? kAngleNaN : (uint32_t)quant_index(angle, PPF_D_ANGLE, 1.0f / PPF_D_ANGLE);
+}
+
+// Index of the three angles of pair_feature, d = p2 - p1 and |d| given.
+__device__ __forceinline__ uint32_t pair_angles(float3 n1, float3 n2, float3 d, float len) {
+  const uint32_t y = angle_index(acosf(dot3(n1, d) / (norm3(n1) * len)));
+  const uint32_t z = angle_index(acosf(dot3(n2, d) / (norm3(n2) * len)));
+  const uint32_t w = angle_index(acosf(dot3(n1, n2) / (norm3(n1) * norm3(n2))));
+  return (y * kAngleValues + z) * kAngleValues + w;
 }
 
 // -------------------------------------------------------- 4x4 transforms --

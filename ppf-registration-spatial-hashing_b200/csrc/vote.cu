@@ -2,19 +2,33 @@
 // (src/cuda/scene.cu:24-55, src/cuda/model.cu:95-171) without materialising
 // scene pair features or individual votes.
 //
-// One work item = (scene reference point s_r, chunk of model reference points).
-// A persistent block (1024 threads, one per SM) takes items from an atomic
-// counter.  For its s_r it walks all scene points in tiles of 1024: each
-// thread computes one pair feature, its FNV key, and looks the key up in the
-// model's key -> run table.  Every matched pair's sub-run (the run entries
-// whose m_r falls in this chunk) is cut into segments of at most 2^seg_shift entries;
-// warps take segments from a shared counter and stream their entries with
-// consecutive lanes on consecutive entries, counting each vote into a
-// shared-memory accumulator of 32-bit (m_r, alpha bin) counters.  When an
-// item is done, the block folds its largest count into a global running
-// maximum and emits every cell whose count exceeds threshold x running
-// maximum: a superset of the cells the final threshold (threshold x global
-// maximum) keeps.
+// One work item = (scene reference point s_r, a range of chunks of model
+// reference points).  A persistent block (1024 threads, one per SM) takes
+// items from an atomic counter.  For its s_r it
+//  1. walks the scene points in tiles of 1024: one pair feature, FNV key and
+//     run lookup per thread; matched pairs ("events") go to a list in shared
+//     memory and are counted per model run in a small hash table,
+//  2. groups the list by run (counting sort) and cuts each group into pieces
+//     of at most kPieceEvents events,
+//  3. per chunk, lets warps take units (a piece x a segment of the run's
+//     entries whose m_r lies in the chunk) and adds their votes to a
+//     shared-memory accumulator of (m_r, alpha bin) counters,
+//  4. folds its largest count into a global running maximum and emits every
+//     cell whose count exceeds threshold x running maximum: a superset of the
+//     cells the final threshold (threshold x global maximum) keeps.
+//
+// Why the grouping: the scene pairs of one s_r fall into few distinct keys
+// (the bench's first model: 2049 matched pairs of 154 keys per s_r, 7.2e7
+// votes but 3.2e6 distinct run entries), so streaming a run once per scene
+// pair reads and counts every entry G times.  A piece of G events adds a
+// whole 30-bin histogram per entry instead (sweep_unit).  Vote pass at
+// ref_point_df 50, a shared atomic per vote against this: 47.1 / 17.7 / 19.5 /
+// 72.8 ms against 23.0 / 12.8 / 13.9 / 19.2 ms for the bench's four models,
+// and 6.7 against 5.9 ms for the 2000-point model and 10000-point scene.  What
+// bounds it now: shared-memory wavefronts of the swept entries (about 53 per
+// 32 entries, two thirds of the time at long sub-runs) and issue slots of the
+// events between them (short sub-runs).
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -25,17 +39,30 @@
 namespace ppf {
 namespace {
 
-// Entries per segment: 1 << VoteArgs::seg_shift.  A warp streams a segment
-// in passes of 256 entries and pays the L2 latency of its first loads and the
-// segment search once per segment; longer segments leave more warps idle at
-// the end of a tile.  Fixed lengths of 1024/2048/4096/8192 measured
-// 57.8/53.2/51.5/51.6 ms on the bench's first model (ref_point_df 50) and
-// 92.1/83.8/79.8/78.3 ms on its fourth: the best length depends on the model,
-// so tune_vote_segments chooses it per model among kSegShifts.
-constexpr uint32_t kSegShifts[] = {11, 12, 13};
-constexpr int kUnroll = 8;        // independent entry loads per lane
 constexpr uint32_t kNoRun = 0xffffffffu;
-constexpr uint32_t kExactOnly = 1u << 31;  // scene angle flag: every vote of the pair takes the exact path
+constexpr uint32_t kExactGroup = 1u << 31;  // group key flag: every vote of its events takes the exact path
+
+// Fixed-point angles: alpha + pi = beta_s - beta_m + 2^20 in 2^-21 turns.
+// With A = 30 x = Q 2^21 + R for x = beta_s + 2^20 (events) and x = beta_m
+// (entries), the bin is Q_s - Q_m - [R_s < R_m] modulo 30, and R_s - R_m
+// modulo 2^21 is the position inside the bin; a vote is ambiguous within
+// kMargin of an edge.
+constexpr uint32_t kTurn = 1u << PPF_ANGLE_BITS;
+constexpr uint32_t kMargin = PPF_BIN_MARGIN_UNITS * PPF_N_ANGLE;
+
+constexpr int kBlock = 128;  // entries of one sub-run that a warp takes at a time
+constexpr int kPerLane = kBlock / 32;
+// A piece of at least kSweepMin events is sorted by R so that it can be swept;
+// it is, where that is cheaper than counting its votes one by one.  Fitted to
+// phase timings of the bench's models, in SM cycles x 32: a counted vote 6.8, a
+// swept entry 40 and an event among its entries 1700, so that sub-runs below
+// 250 entries are always counted and long ones swept from 7 events on.
+constexpr uint32_t kSweepMin = 7;
+__device__ __forceinline__ bool sweep_pays(uint32_t events, uint32_t entries) {
+  return events >= kSweepMin && 7.f * (float)events * (float)entries > 40.f * (float)entries + 1700.f * (float)events;
+}
+// A chunk's units are halved, down to 512 entries, until there are this many.
+constexpr uint32_t kMinUnits = 256, kMinUnitShift = 9;
 
 struct VoteArgs {
   // model
@@ -47,11 +74,17 @@ struct VoteArgs {
   const uint32_t* ht_keys;
   const uint32_t* ht_runs;
   uint32_t ht_mask;
+  const uint32_t* lut;        // ModelTables::lut, or null: every scene pair is hashed
+  const uint32_t* row_flags;
   const float4* m_r1;
   const float4* m_r2;
   const float4* m_pts;
   uint32_t n_m, chunk, n_chunks;
-  uint32_t seg_shift;  // log2 of the segment length
+  const uint32_t* run_maxl;  // per run: most entries that share one m_r
+  uint32_t unit_shift;  // log2 of the entries per unit
+  uint32_t r_shift;     // entries of a sub-run are in ascending order of R >> r_shift
+  uint32_t cpi, n_cg;   // chunks per work item, work items per scene reference point
+  uint2* spill;         // per block: 32-bit counts of a chunk's cells (see spill_acc)
   // scene
   const float4* s_pts;
   const float4* s_nrm;
@@ -126,32 +159,43 @@ __device__ __forceinline__ void block_sync() {
   __threadfence_block();
 }
 
-// Exclusive block scan of one value per thread; `total` receives the sum.
-// s_warp is this call site's own 32-word scratch; the caller places a barrier
-// between two scans on the same scratch (both call sites have several).
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+// Exclusive block scans of one or two values per thread; the totals come
+// back by reference.  s_warp is this call site's own scratch; the caller
+// places a barrier between two scans on the same scratch.
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
+  return x;
+}
+
+__device__ __forceinline__ uint2 block_excl_scan(uint2 v, uint2* s_warp, uint2& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint2 x = make_uint2(warp_incl_scan(v.x), warp_incl_scan(v.y));
   if (lane == 31) s_warp[warp] = x;
   block_sync();
   if (warp == 0) {
-    uint32_t w = s_warp[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    s_warp[lane] = w;
+    const uint2 w = s_warp[lane];
+    s_warp[lane] = make_uint2(warp_incl_scan(w.x), warp_incl_scan(w.y));
   }
   block_sync();
-  const uint32_t r = (warp ? s_warp[warp - 1] : 0u) + x - v;
+  const uint2 below = warp ? s_warp[warp - 1] : make_uint2(0u, 0u);
   total = s_warp[kVoteWarps - 1];
-  return r;
+  return make_uint2(below.x + x.x - v.x, below.y + x.y - v.y);
+}
+
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t x = warp_incl_scan(v);
+  if (lane == 31) s_warp[warp] = x;
+  block_sync();
+  if (warp == 0) s_warp[lane] = warp_incl_scan(s_warp[lane]);
+  block_sync();
+  total = s_warp[kVoteWarps - 1];
+  return (warp ? s_warp[warp - 1] : 0u) + x - v;
 }
 
 // Exact bin of one vote: the reference's own arithmetic for it.  The model
@@ -171,20 +215,81 @@ __device__ __forceinline__ uint32_t exact_bin(const VoteArgs& a, uint32_t pos, f
   return alpha_bin_exact(u, v);
 }
 
-// Per-block shared state of a vote kernel besides the dynamic queue and
-// accumulator.
+// ---- shared-memory layout of a vote block (dynamic allocation, 32-bit words)
+//
+// Events of one s_r held at a time; a walk that fills the list is continued
+// after its votes are counted.  A warp looks up 32 pairs only while at most
+// kGroupLimit groups exist, so that all warps' pairs fit the slots.
+constexpr uint32_t kEvents = 7168;
+constexpr uint32_t kEventsPerThread = kEvents / kVoteThreads;
+constexpr uint32_t kSlots = 2048;
+constexpr uint32_t kGroupLimit = 640;
+constexpr uint32_t kPieceEvents = 255;  // a histogram counter fits a byte
+constexpr uint32_t kMaxPieces = kGroupLimit + kVoteThreads + (kEvents + kPieceEvents - 1) / kPieceEvents;
+static_assert(kGroupLimit + kVoteThreads < kSlots, "every warp's groups find a slot");
+static_assert(kMaxPieces <= 2 * kVoteThreads, "two pieces per thread");
+static_assert(4 * (kMaxPieces + 1) <= kEvents, "per-chunk piece arrays fit the event slot words");
+
+constexpr uint32_t kOffEvW = 0;                          // A = Q << 21 | R of each event
+constexpr uint32_t kOffEvI = kOffEvW + kEvents;          // its scene point
+constexpr uint32_t kOffEvK = kOffEvI + kEvents;          // slot << 16 | rank in the group, until grouped
+constexpr uint32_t kOffSlotKey = kOffEvK + kEvents;      // run | kExactGroup
+constexpr uint32_t kOffSlotCnt = kOffSlotKey + kSlots;   // events, then offset of the group
+constexpr uint32_t kOffPcRun = kOffSlotCnt + kSlots;     // piece: its run
+constexpr uint32_t kOffPcInf = kOffPcRun + kMaxPieces;   // piece: see piece_info
+constexpr uint32_t kOffAcc = (kOffPcInf + kMaxPieces + 31) / 32 * 32;  // counters, see kRowStride
+// over the pieces while the list is filled: per warp the scene pairs that
+// await their lookup
+constexpr uint32_t kNearLen = 64;
+constexpr uint32_t kOffNear = kOffPcRun;
+static_assert(kVoteWarps * kNearLen <= 2 * kMaxPieces, "the waiting pairs fit the pieces");
+// over the event slot words once the list is grouped: the pieces' entries in
+// the current chunk (first entry, length, first unit, running counter bound)
+constexpr uint32_t kOffPcLo = kOffEvK;
+constexpr uint32_t kOffPcLen = kOffPcLo + kMaxPieces + 1;
+constexpr uint32_t kOffPcUnit = kOffPcLen + kMaxPieces + 1;
+constexpr uint32_t kOffPcInc = kOffPcUnit + kMaxPieces + 1;
+// over the slots once the list is grouped: per warp a histogram table and a
+// queue of ambiguous votes
+constexpr uint32_t kTabWords = 60, kQueueLen = 32;
+constexpr uint32_t kOffTab = kOffSlotKey;
+constexpr uint32_t kOffQueue = kOffTab + kVoteWarps * kTabWords;
+static_assert(kVoteWarps * (kTabWords + 2 * kQueueLen) <= 2 * kSlots, "tables and queues fit the slots");
+
+// Accumulator: plane j holds the 16-bit counters of bins (2j, 2j + 1) of every
+// m_r of the chunk, one word each, and a last plane the 32-bit counters of
+// bin 30 (only alpha == pi exactly reaches it).  The planes are a multiple of
+// 32 words apart, so a counter's bank is its m_r mod 32 whatever the bin, and
+// 32 lanes with distinct m_r mod 32 count without bank conflicts.
+constexpr uint32_t kPlanes = PPF_N_ANGLE / 2;
+constexpr uint32_t kRowStride = (kMaxChunk + 31) / 32 * 32;
+// A row no chunk has: lanes past a sub-run's end count there, so that the
+// adds need no branch.  Never read.
+constexpr uint32_t kPadRow = kRowStride - 1;
+static_assert(kPadRow >= kMaxChunk && kPadRow < (1u << (32 - PPF_ANGLE_BITS)), "a spare row in every plane");
+constexpr uint32_t kCounterMax = 65535;
+
+// uint2 counters that a block spills to (spill_acc)
+constexpr size_t kSpillWords = (size_t)kPlanes * kRowStride;
+constexpr size_t kVoteSmemBytes = (size_t)(kOffAcc + (kPlanes + 1) * kRowStride) * 4;
+
+// pc_inf: first event (13 bits) | events (8) | exact (1) | largest histogram
+// window (8, see sort_piece)
+__device__ __forceinline__ uint32_t piece_info(uint32_t off, uint32_t cnt, bool exact, uint32_t win) {
+  return off | cnt << 13 | (exact ? 1u << 21 : 0u) | win << 22;
+}
+
+// Per-block shared state of a vote kernel besides the dynamic allocation.
 struct VoteShared {
   // the item's scene reference point, its normal and rows 1-2 of its frame:
   // read from here by the scene walk of each tile, so that they do not hold
   // 14 registers through the vote passes between walks
   float4 p_r, n_r, f_r1, f_r2;
   uint32_t item, next, max, base;
-  uint32_t scan_seg[kVoteWarps];   // scratch of the per-tile segment scan
+  uint32_t n_ev, n_gr;  // events and groups of the list
+  uint32_t rows[kFlagRows / 32];  // the model's row flags
+  uint2 scan2[kVoteWarps];         // scratch of the two-value scans
   uint32_t scan_emit[kVoteWarps];  // scratch of the emission scan
-  // q_seg at the first pair of each warp's 32 (q_seg[32 l]), kept
-  // contiguous: the segment search reads all 32 in one conflict-free access
-  // (read in place they sit in one bank, 32 accesses per search)
-  uint32_t seg_blk[kVoteWarps];
   uint32_t wmax[kVoteWarps];       // per-warp maxima of the accumulator
 };
 
@@ -220,304 +325,940 @@ __device__ __forceinline__ uint32_t fetch_item(uint32_t* work_counter, VoteShare
   return sh.item;
 }
 
-// One work item (s_r, chunk) of request `a`: slot_of_item indexes a's items
-// (or a.item_list).  Called by every thread of the block.
+extern __shared__ __align__(16) uint32_t smem[];
+
+// The warp's histogram table and queue.
+__device__ __forceinline__ uint32_t* warp_tab() { return smem + kOffTab + (threadIdx.x >> 5) * kTabWords; }
+__device__ __forceinline__ uint32_t* warp_queue() { return smem + kOffQueue + (threadIdx.x >> 5) * 2 * kQueueLen; }
+
+__device__ __forceinline__ uint32_t wrap30(int b) { return (uint32_t)(b < 0 ? b + PPF_N_ANGLE : b); }
+
+// y' of an event word A and an entry: alpha + pi in 2^-32 turns, shifted down
+// by the ambiguity margin (the entry's row bits shift out).
+constexpr int kAngleShift = 32 - PPF_ANGLE_BITS;
+__device__ __forceinline__ uint32_t count_angle(uint32_t w, uint32_t entry) {
+  return ((w / PPF_N_ANGLE - PPF_BIN_MARGIN_UNITS) << kAngleShift) - (entry << kAngleShift);
+}
+
+// One vote more in (row, bin).
+__device__ __forceinline__ void add_cell(uint32_t row, uint32_t bin) {
+  uint32_t* const acc = smem + kOffAcc + row;
+  if (bin == PPF_N_ANGLE) atomicAdd(acc + kPlanes * kRowStride, 1u);
+  else atomicAdd(acc + (bin >> 1) * kRowStride, 1u << (16 * (bin & 1)));
+}
+
+// One vote less in (row, bin), bin < 30; the vote was counted there before,
+// so the 16-bit counter does not borrow.
+__device__ __forceinline__ void sub_cell(uint32_t row, uint32_t bin) {
+  atomicSub(smem + kOffAcc + row + (bin >> 1) * kRowStride, 1u << (16 * (bin & 1)));
+}
+
+// Votes near a bin edge are counted in a provisional bin and queued per warp:
+// (entry, event | provisional bin << 16).  A full queue is binned by the
+// reference's exact arithmetic, one vote per lane: the exact path's loads and
+// atan2f then run for 32 votes at once (they are 1.7e-4 of all votes, and
+// one at a time they cost as much as the sweep itself).
 template <bool kCheck>
-__device__ __forceinline__ void vote_item(const VoteArgs& a, uint32_t slot_of_item, VoteShared& sh,
-                                          VoteStats& st) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  uint32_t* q_lo = smem;                        // [kVoteThreads]
-  uint32_t* q_len = q_lo + kVoteThreads;        // [kVoteThreads]
-  uint32_t* q_beta = q_len + kVoteThreads;      // [kVoteThreads]
-  float2* q_v = reinterpret_cast<float2*>(q_beta + kVoteThreads);       // [kVoteThreads]
-  uint32_t* q_seg = reinterpret_cast<uint32_t*>(q_v + kVoteThreads);    // [kVoteThreads + 4]
-  uint32_t* acc = q_seg + kVoteThreads + 4;
+__device__ __forceinline__ void drain_queue(const VoteArgs& a, const VoteShared& sh, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t* const queue = warp_queue();
+  __syncwarp();
+  if (lane < n) {
+    const uint32_t pos = queue[2 * lane], inf = queue[2 * lane + 1];
+    const uint32_t fast = inf >> 16;
+    uint32_t i = in_range<kCheck>(a, 17, inf & 0xffffu, kEvents) ? smem[kOffEvI + (inf & 0xffffu)] : 0u;
+    if (!in_range<kCheck>(a, 18, i, a.n_s)) i = 0;
+    const float4 p4 = a.s_pts[i];
+    FrameYZ fs;
+    fs.r1 = sh.f_r1;
+    fs.r2 = sh.f_r2;
+    const uint32_t exact = exact_bin<kCheck>(a, pos, frame_point_yz(fs, make_float3(p4.x, p4.y, p4.z)));
+    if (exact != fast && in_range<kCheck>(a, 19, fast, PPF_N_ANGLE) && in_range<kCheck>(a, 23, pos, a.P)) {
+      const uint32_t row = __ldg(a.entries + pos) >> PPF_ANGLE_BITS;
+      if (in_range<kCheck>(a, 7, row, a.chunk)) {
+        sub_cell(row, fast);
+        add_cell(row, exact);
+      }
+    }
+  }
+  __syncwarp();
+}
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t cells = a.chunk * kBins;
-  const uint32_t seg_len = 1u << a.seg_shift;
-  {
-    const uint32_t item = a.item_list ? a.item_list[slot_of_item] : slot_of_item;
-    const uint32_t c = item % a.n_chunks;
-    // ref < n_ref, so sr = ref * ref_df < n_s
-    const uint32_t ref = (uint32_t)(((unsigned long long)(item / a.n_chunks) * a.perm_mul) % a.n_ref);
-    const uint32_t sr = ref * a.ref_df;
-    const uint32_t mr_lo = c * a.chunk;
-    // thread 0 publishes the frame of s_r; the barrier after the clear makes
-    // it visible, and the previous item's readers are past the item-fetch
-    // barrier before it is overwritten
-    if (tid == 0) {
-      const float4 p4 = a.s_pts[sr], n4 = a.s_nrm[sr];
-      const FrameYZ f = frame_yz(make_float3(p4.x, p4.y, p4.z), make_float3(n4.x, n4.y, n4.z));
-      sh.p_r = p4;
-      sh.n_r = n4;
-      sh.f_r1 = f.r1;
-      sh.f_r2 = f.r2;
+// Queues the ambiguous votes of one event among the block's entries at pos
+// (bit k of a lane's mask: its k-th entry) and returns the queue's new length.
+// Called by the whole warp; it is rare and recomputes from the entries what
+// its callers hold in registers.
+template <bool kCheck>
+__device__ __forceinline__ uint32_t queue_votes(const VoteArgs& a, const VoteShared& sh, uint32_t mask, uint32_t pos,
+                                             uint32_t ev, bool sweep, uint32_t qn) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t w = smem[kOffEvW + ev];
+  uint32_t* const queue = warp_queue();
+#pragma unroll 1
+  for (int k = 0; k < kPerLane; ++k) {
+    const bool amb = mask >> k & 1u;
+    const uint32_t lanes = __ballot_sync(0xffffffffu, amb);
+    if (!lanes) continue;
+    const uint32_t n = __popc(lanes);
+    if (qn + n > kQueueLen) {
+      drain_queue<kCheck>(a, sh, qn);
+      qn = 0;
     }
-    for (uint32_t i = tid; i < cells; i += kVoteThreads) acc[i] = 0u;
-    block_sync();
+    if (amb && in_range<kCheck>(a, 27, pos + 32u * k + lane, a.P)) {
+      const uint32_t at = qn + __popc(lanes & ((1u << lane) - 1u));
+      const uint32_t e = __ldg(a.entries + pos + 32u * k + lane);
+      uint32_t bin;
+      if (sweep) {
+        const uint32_t t = (e & (kTurn - 1u)) * PPF_N_ANGLE;
+        const int below = (w & (kTurn - 1u)) < (t & (kTurn - 1u)) ? 1 : 0;
+        bin = wrap30((int)(w >> PPF_ANGLE_BITS) - (int)(t >> PPF_ANGLE_BITS) - below);
+      } else {
+        bin = (uint32_t)((unsigned long long)count_angle(w, e) * PPF_N_ANGLE >> 32);
+      }
+      queue[2 * at] = pos + 32u * k + lane;
+      queue[2 * at + 1] = ev | bin << 16;
+    }
+    qn += n;
+  }
+  __syncwarp();
+  return qn;
+}
 
-    for (uint32_t base = 0; base < a.n_s; base += kVoteThreads) {
-      // ---- one scene pair per thread: feature, key, lookup, sub-run
-      const uint32_t i = base + tid;
-      uint32_t len = 0, lo = 0, beta = 0;
-      float2 v = make_float2(0.f, 0.f);
-      if (i < a.n_s && i != sr) {
-        float4 pi4 = a.s_pts[i], ni4 = a.s_nrm[i];
-        float3 pi = make_float3(pi4.x, pi4.y, pi4.z);
-        const float4 p4 = sh.p_r, n4 = sh.n_r;
-        float4 f = pair_feature(make_float3(p4.x, p4.y, p4.z), make_float3(n4.x, n4.y, n4.z), pi,
-                                make_float3(ni4.x, ni4.y, ni4.z), a.d_dist);
-        uint32_t key = feature_key(f);
-        if (key != 0u) {
-          uint32_t run = ht_lookup(a.ht_keys, a.ht_runs, a.ht_mask, key);
-          if (run != kNoRun && in_range<kCheck>(a, 2, run, a.K)) {
-            const uint32_t* sp = a.split + (size_t)run * (a.n_chunks + 1);
-            lo = __ldg(sp + c);
-            len = __ldg(sp + c + 1) - lo;
-            if (kCheck && !in_range<kCheck>(a, 3, (unsigned long long)lo + len, a.P + 1)) len = 0;
-            if (c == 0 && !a.item_list) {
-              st.votes += __ldg(a.run_count + run);
-              st.matched += 1;
-            }
-            if (len) {
-              FrameYZ fs;
-              fs.r1 = sh.f_r1;
-              fs.r2 = sh.f_r2;
-              v = frame_point_yz(fs, pi);
-              bool degenerate = fabsf(v.x) + fabsf(v.y) < 1e-12f || !isfinite(v.x) || !isfinite(v.y);
-              beta = angle21(v) | ((degenerate || __ldg(a.run_flags + run)) ? kExactOnly : 0u);
-            }
-          }
-        }
-      }
-      uint32_t n_seg_total;
-      const uint32_t seg0 = block_excl_scan((len + seg_len - 1) >> a.seg_shift, sh.scan_seg, n_seg_total);
-      q_lo[tid] = lo;
-      q_len[tid] = len;
-      q_beta[tid] = beta;
-      q_v[tid] = v;
-      q_seg[tid] = seg0;
-      if (lane == 0) sh.seg_blk[warp] = seg0;
-      if (tid == 0) {
-        q_seg[kVoteThreads] = n_seg_total;
-        sh.next = kVoteWarps;
-      }
-      block_sync();
-      if (kCheck) {
-        const uint32_t want = q_seg[tid] + ((q_len[tid] + seg_len - 1) >> a.seg_shift);
-        if (q_seg[tid] != seg0 || q_seg[tid + 1] != want)
-          in_range<kCheck>(a, 11, ((unsigned long long)tid << 32) | q_seg[tid + 1], want);
-      }
-
-      // ---- warps take segments; lanes stream consecutive entries
-      uint32_t s = warp;
-      while (s < n_seg_total) {
-        // pair p with q_seg[p] <= s < q_seg[p+1]: the last index whose segment
-        // offset is <= s (q_seg is nondecreasing and q_seg[0] = 0), found with
-        // two ballots: first over q_seg[32 l] (its copy seg_blk[l]), then
-        // inside that block of 32
-        const uint32_t blk = 31u - __clz(__ballot_sync(0xffffffffu, sh.seg_blk[lane] <= s));
-        const uint32_t plo = 32u * blk + 31u - __clz(__ballot_sync(0xffffffffu, q_seg[32 * blk + lane] <= s));
-        const uint32_t p = plo;
-        const uint32_t start = q_lo[p] + ((s - q_seg[p]) << a.seg_shift);
-        uint32_t end = min(q_lo[p] + q_len[p], start + seg_len);
-        // Always-on guard (one compare per segment of up to 1024 votes): a
-        // segment outside its sub-run or the entry array is recorded, raises
-        // kFlagBadIndex and is skipped, so the lookup fails instead of the
-        // kernel reading outside the entries.
-        if (start >= end || end > a.P) {
-          if (lane == 0) {
-            if (atomicCAS(&a.bad[3], 0ull, 1ull) == 0ull) {
-              a.bad[4] = ((unsigned long long)p << 32) | s;
-              a.bad[5] = ((unsigned long long)q_seg[p] << 32) | q_seg[p + 1];
-              a.bad[6] = ((unsigned long long)q_lo[p] << 32) | q_len[p];
-              a.bad[7] = ((unsigned long long)n_seg_total << 32) | q_seg[kVoteThreads];
-              a.bad[8] = ((unsigned long long)base << 32) | item;
-              a.bad[9] = ((unsigned long long)warp << 32) | plo;
-            }
-            atomicOr(a.flags, (uint32_t)kFlagBadIndex);
-          }
-          end = start;
-        }
-        const uint32_t bw = q_beta[p];
-        const float2 vv = q_v[p];
-        // Each entry holds the pair's m_r inside the chunk in its top 11 bits
-        // and the model angle beta_m in its low 21.  With y = (beta_s + 2^20 -
-        // beta_m) << 11, i.e. alpha + pi in 2^-32 turns (the row bits and the
-        // exact-only flag shift out), the bin is the high word of y * 30 and
-        // the low word the position inside the bin; a vote is ambiguous when
-        // that position is within the margin m = 6 units of an edge.  One
-        // 32 x 32 -> 64 multiply gives both words of the margin-shifted angle
-        // y' = y - m:  30 y' = 30 y - 30 m, so a vote is unambiguous exactly
-        // when the low word of 30 y' is at most m_span, and its high word is
-        // then the bin of y.  For the ambiguous votes the high word is still
-        // in [0, 29] (y' wraps to 2^32 + y - m only when 30 y < 30 m, giving
-        // 29), so their provisional fast cell stays inside the accumulator.
-        constexpr int kShift = 32 - PPF_ANGLE_BITS;
-        const uint32_t bsh = ((bw + (1u << (PPF_ANGLE_BITS - 1))) << kShift) -
-                             ((uint32_t)PPF_BIN_MARGIN_UNITS << kShift);
-        constexpr uint32_t m_span =
-            ((1u << PPF_ANGLE_BITS) - 2 * PPF_BIN_MARGIN_UNITS * PPF_N_ANGLE) << kShift;
-        // (bin, position) of a margin-shifted angle: high and low word of 30 y'
-        auto bin_pos = [](uint32_t yp) { return (unsigned long long)yp * (uint32_t)PPF_N_ANGLE; };
-        const uint32_t* ep = a.entries + start + lane;
-        const uint32_t n_here = end - start;
-        // Votes near a bin edge were counted in their fast cell; move them to
-        // the cell of the reference's exact arithmetic (rare: ~1.7e-4 of
-        // votes).  The pass's entries are still in registers (c), so only the
-        // exact path's own loads remain; pass_pos is the position of this
-        // lane's first entry of the pass.
-        auto fix_up = [&](uint32_t pass_pos, const uint32_t(&c)[kUnroll]) {
-          uint32_t mask = 0;
+// Entries [pos, pos + 128) of a unit that ends at `end`, kPerLane per lane
+// (the pad row past the end).
+__device__ __forceinline__ void load_block(const uint32_t* entries, uint32_t pos, uint32_t end,
+                                           uint32_t (&e)[kPerLane]) {
+  const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
-          for (int u = 0; u < kUnroll; ++u)
-            if ((uint32_t)bin_pos(bsh - (c[u] << kShift)) > m_span) mask |= 1u << u;
-          while (mask) {
-            const int u = __ffs(mask) - 1;
-            mask &= mask - 1;
-            uint32_t e = c[0];
-#pragma unroll
-            for (int k = 1; k < kUnroll; ++k) e = (u == k) ? c[k] : e;
-            const uint32_t pos = pass_pos + 32u * (uint32_t)u;
-            const unsigned long long bp = bin_pos(bsh - (e << kShift));
-            const uint32_t row = (e >> PPF_ANGLE_BITS) * kBins;
-            const uint32_t fast = row + (uint32_t)(bp >> 32);
-            const uint32_t exact = row + exact_bin<kCheck>(a, pos, vv);
-            if (exact != fast && in_range<kCheck>(a, 7, exact, cells)) {
-              atomicAdd(&acc[fast], 0xffffffffu);
-              atomicAdd(&acc[exact], 1u);
-            }
-            ++st.exact;
-          }
-        };
-        if (bw & kExactOnly) {
-          // degenerate frame vector or run: every vote takes the exact path
-          for (uint32_t k = lane; k < n_here; k += 32) {
-            const uint32_t row = (__ldg(a.entries + start + k) >> PPF_ANGLE_BITS) * kBins;
-            const uint32_t cell = row + exact_bin<kCheck>(a, start + k, vv);
-            if (in_range<kCheck>(a, 6, cell, cells)) atomicAdd(&acc[cell], 1u);
-            ++st.exact;
-          }
-        } else {
-          // kUnroll entries per lane per pass, branch-free: the fast cell of
-          // every vote is counted, and the rare votes near a bin edge are
-          // moved afterwards.  The last pass is masked to the segment's end.
-          const uint32_t nfull = n_here / (32 * kUnroll);
-          for (uint32_t it = 0; it < nfull; ++it, ep += 32 * kUnroll) {
-            uint32_t c[kUnroll];
-            bool amb = false;
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) c[u] = __ldg(ep + 32 * u);
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-              const unsigned long long bp = bin_pos(bsh - (c[u] << kShift));
-              amb |= (uint32_t)bp > m_span;
-              const uint32_t cell = (c[u] >> PPF_ANGLE_BITS) * kBins + (uint32_t)(bp >> 32);
-              if (in_range<kCheck>(a, 8, cell, cells)) atomicAdd(&acc[cell], 1u);
-            }
-            if (amb) fix_up(start + it * 32u * kUnroll + lane, c);
-          }
-          for (uint32_t k = nfull * 32 * kUnroll + lane; k < n_here; k += 32) {
-            const uint32_t e = __ldg(a.entries + start + k);
-            const unsigned long long bp = bin_pos(bsh - (e << kShift));
-            uint32_t cell = (e >> PPF_ANGLE_BITS) * kBins + (uint32_t)(bp >> 32);
-            if ((uint32_t)bp > m_span) {
-              cell = (e >> PPF_ANGLE_BITS) * kBins + exact_bin<kCheck>(a, start + k, vv);
-              ++st.exact;
-            }
-            if (in_range<kCheck>(a, 8, cell, cells)) atomicAdd(&acc[cell], 1u);
-          }
-        }
-        if (lane == 0) s = atomicAdd(&sh.next, 1u);
-        s = __shfl_sync(0xffffffffu, s, 0);
-      }
-      if (kCheck && (q_seg[tid] != seg0 || q_len[tid] != len || q_lo[tid] != lo))
-        in_range<kCheck>(a, 12, ((unsigned long long)tid << 32) | q_seg[tid], seg0);
-      // No barrier here: the next tile writes the queue only after the two
-      // barriers of its segment scan, which every warp reaches after its
-      // last segment.
-    }
-    block_sync();  // all votes of the item are counted
-
-    // ---- running maximum, emission
-    uint32_t lmax = 0;
-    for (uint32_t w = tid; w < cells; w += kVoteThreads) lmax = max(lmax, acc[w]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
-    if (lane == 0) sh.wmax[warp] = lmax;
-    block_sync();
-    if (warp == 0) {
-      uint32_t m = sh.wmax[lane];
-#pragma unroll
-      for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-      uint32_t old = 0;
-      if (lane == 0) old = atomicMax(a.global_max, m);
-      old = __shfl_sync(0xffffffffu, old, 0);
-      if (lane == 0) sh.max = max(old, m);
-    }
-    block_sync();
-    const float floor_v = a.floor >= 0.f ? a.floor : a.thr * (float)sh.max;
-    // All-or-nothing slot reservation for the item's cells: an item that does
-    // not fit writes nothing and is queued for a second launch after the
-    // buffer has grown, so the buffer never holds a partial item.
-    uint32_t my_n = 0;
-    for (uint32_t cell = tid; cell < cells; cell += kVoteThreads) {
-      const uint32_t cnt = acc[cell];
-      my_n += (cnt != 0u && (a.emit_all || (float)cnt > floor_v)) ? 1u : 0u;
-    }
-    uint32_t item_total;
-    const uint32_t my_off = block_excl_scan(my_n, sh.scan_emit, item_total);
-    if (warp == 0) {
-      // The whole warp walks the reservation loop in lockstep (lane 0 issues
-      // the atomics, every exit condition is warp-uniform).
-      uint32_t base_slot = 0xffffffffu;
-      if (item_total) {
-        if (lane == 0) atomicAdd(a.n_needed, (unsigned long long)item_total);
-        uint32_t old = 0;
-        if (lane == 0) old = *(volatile uint32_t*)a.n_cand;
-        old = __shfl_sync(0xffffffffu, old, 0);
-        for (int tries = 0; tries < (1 << 20); ++tries) {
-          if ((unsigned long long)old + item_total > a.cand_cap) break;
-          uint32_t prev = 0;
-          if (lane == 0) prev = atomicCAS(a.n_cand, old, old + item_total);
-          prev = __shfl_sync(0xffffffffu, prev, 0);
-          if (prev == old) {
-            base_slot = old;
-            break;
-          }
-          old = prev;
-        }
-        if (base_slot == 0xffffffffu && lane == 0) {
-          const uint32_t k = atomicAdd(a.n_redo, 1u);
-          if (in_range<kCheck>(a, 9, k, a.n_items_total)) a.redo_items[k] = item;
-        }
-      }
-      if (lane == 0) sh.base = base_slot;
-    }
-    block_sync();
-    const uint32_t item_base = sh.base;
-    if (item_base != 0xffffffffu) {
-      uint32_t slot = item_base + my_off;
-      for (uint32_t cell = tid; cell < cells; cell += kVoteThreads) {
-        const uint32_t cnt = acc[cell];
-        if (cnt != 0u && (a.emit_all || (float)cnt > floor_v)) {
-          const uint32_t mr = mr_lo + cell / kBins, bin = cell % kBins;
-          if (in_range<kCheck>(a, 10, slot, a.cand_cap)) {
-            a.cand_code[slot] = ((unsigned long long)sr << 32) | ((unsigned long long)mr << 6) | bin;
-            a.cand_count[slot] = cnt;
-          }
-          ++slot;
-        }
-      }
-    }
-    // The item-fetch barrier of the caller separates these reads of the
-    // accumulator from the next item's clear.
+  for (int k = 0; k < kPerLane; ++k) {
+    const uint32_t p = pos + 32u * k + lane;
+    e[k] = p < end ? __ldg(entries + p) : kPadRow << PPF_ANGLE_BITS;
   }
 }
 
+// A unit of a piece that is swept (sweep_pays): entries [start, end) of
+// the piece's sub-run against events [ev0, ev0 + cnt), in ascending R.
+//
+// The votes of one entry (Q_m, R_m, row) are the histogram
+// H[k] = #{events: Q_s - [R_s < R_m] = k}, rotated by Q_m: 30 counters for
+// any number of events.  The entries come in ascending R (by buckets of
+// 2^r_shift), so H changes only as R_m passes an event.  Per block of 128
+// entries the warp keeps H as of the block's first bucket in a table of
+// packed quadruples H[k .. k + 3], k = 0..59 modulo 30, and every lane adds it
+// to its entry's row: it reads the 8 table words Q_m + 4j (the lanes' words
+// lie among 30 consecutive ones: distinct banks or one broadcast) and adds 15
+// words of 16-bit pairs, one per plane.  Events that lie inside the block's
+// bucket range then move one vote for each entry beyond them.  Returns the
+// queue's length and the lane's ambiguous votes.  Out of line and without
+// calls of its own (as count_unit), so that neither the block's phases around
+// it nor a callee's saved registers spill in its loops.
 template <bool kCheck>
-__global__ void __launch_bounds__(kVoteThreads, 1) vote_kernel(VoteArgs a) {
+__device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh, uint32_t start, uint32_t end,
+                                           uint32_t ev0, uint32_t cnt, uint32_t qn) {
+  uint32_t n_exact = 0;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t* const ev = smem + kOffEvW + ev0;
+  uint32_t* const acc = smem + kOffAcc;
+  uint32_t* const tab = warp_tab();
+  const uint32_t rs = a.r_shift;
+  const uint32_t* const entries = a.entries;  // (a copy: a's fields are read anew after every atomic)
+  uint32_t passed = 0;  // events of a bucket below the block's first: counted in H as Q_s - 1
+  uint32_t done = 0;    // events too far below the block's first bucket to be ambiguous in it or later
+  uint32_t h = 0;       // H[lane]
+  for (uint32_t pos = start; pos < end; pos += kBlock) {
+    const uint32_t n = min((uint32_t)kBlock, end - pos);
+    int rm[kPerLane];  // R_m (-kTurn past the end: below every event)
+    uint32_t row[kPerLane], qm[kPerLane];
+    uint32_t rmin = kTurn, rmax = 0;
+    uint32_t e[kPerLane];
+    load_block(entries, pos, end, e);
+#pragma unroll
+    for (int k = 0; k < kPerLane; ++k) {
+      const uint32_t t = (e[k] & (kTurn - 1u)) * PPF_N_ANGLE;
+      const bool valid = 32u * k + lane < n;
+      rm[k] = valid ? (int)(t & (kTurn - 1u)) : -(int)kTurn;
+      row[k] = e[k] >> PPF_ANGLE_BITS;
+      qm[k] = t >> PPF_ANGLE_BITS;
+      if (valid) {
+        rmin = min(rmin, (uint32_t)rm[k]);
+        rmax = max(rmax, (uint32_t)rm[k]);
+      }
+    }
+    rmin = __reduce_min_sync(0xffffffffu, rmin);
+    rmax = __reduce_max_sync(0xffffffffu, rmax);
+    const uint32_t b0 = rmin >> rs, b1 = rmax >> rs;
+    bool changed = false;
+    if (pos == start) {
+      tab[lane] = 0u;
+      __syncwarp();
+      for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
+        bool below = false, far = false;
+        if (j0 + lane < cnt) {
+          const uint32_t w = ev[j0 + lane], r = w & (kTurn - 1u), q = w >> PPF_ANGLE_BITS;
+          below = (r >> rs) < b0;
+          far = r + kMargin <= b0 << rs;
+          atomicAdd(tab + (below ? (q ? q - 1u : PPF_N_ANGLE - 1u) : q), 1u);
+        }
+        passed += __popc(__ballot_sync(0xffffffffu, below));
+        done += __popc(__ballot_sync(0xffffffffu, far));
+      }
+      __syncwarp();
+      h = tab[lane];
+      changed = true;
+    } else {
+      while (passed < cnt) {
+        const uint32_t w = ev[passed], q = w >> PPF_ANGLE_BITS;
+        if (((w & (kTurn - 1u)) >> rs) >= b0) break;
+        h += (lane == (q ? q - 1u : PPF_N_ANGLE - 1u) ? 1u : 0u) - (lane == q ? 1u : 0u);
+        changed = true;
+        ++passed;
+      }
+      while (done < cnt && (ev[done] & (kTurn - 1u)) + kMargin <= b0 << rs) ++done;
+    }
+    if (changed) {
+      const uint32_t k1 = lane + 1 >= PPF_N_ANGLE ? lane + 1 - PPF_N_ANGLE : lane + 1;
+      const uint32_t k2 = lane + 2 >= PPF_N_ANGLE ? lane + 2 - PPF_N_ANGLE : lane + 2;
+      const uint32_t two = h | __shfl_sync(0xffffffffu, h, k1) << 8;
+      const uint32_t four = two | __shfl_sync(0xffffffffu, two, k2) << 16;
+      __syncwarp();
+      if (lane < PPF_N_ANGLE) {
+        tab[lane] = four;
+        tab[lane + PPF_N_ANGLE] = four;
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < kPerLane; ++k) {
+      if (32u * k < n && in_range<kCheck>(a, 8, row[k], kRowStride)) {
+        const uint32_t* const tp = tab + qm[k];
+        uint32_t* const ap = acc + row[k];
+        uint32_t v[(kPlanes + 1) / 2];
+#pragma unroll
+        for (uint32_t j = 0; j < (kPlanes + 1) / 2; ++j) v[j] = tp[4 * j];
+#pragma unroll
+        for (uint32_t j = 0; j < kPlanes; ++j)
+          atomicAdd(ap + j * kRowStride, __byte_perm(v[j / 2], 0u, j & 1 ? 0x4342 : 0x4140));
+      }
+    }
+    __syncwarp();
+    // events among the block's entries, and within the margin of one; a block
+    // near R = 0 meets the margin across it and looks at every event
+    const bool edge = rmin < kMargin || rmax > kTurn - kMargin;
+    for (uint32_t q = edge ? 0u : min(passed, done); q < cnt; ++q) {
+      const uint32_t w = ev[q], re = w & (kTurn - 1u), qe = w >> PPF_ANGLE_BITS;
+      if (!edge && (re >> rs) > b1 && re >= rmax + kMargin) break;
+      uint32_t nearest = kTurn;  // distance above the margin's lower end, modulo a bin
+#pragma unroll
+      for (int k = 0; k < kPerLane; ++k)
+        nearest = min(nearest, (uint32_t)((int)re - rm[k] + (int)kMargin - 1) & (kTurn - 1u));
+      if (q >= passed) {
+#pragma unroll
+        for (int k = 0; k < kPerLane; ++k) {
+          if ((int)re < rm[k] && in_range<kCheck>(a, 13, row[k], a.chunk)) {
+            // (unsigned minima wrap the bins: below 0 is a large number)
+            const uint32_t d = qe - qm[k], b = min(d, d + PPF_N_ANGLE), to = min(b - 1u, PPF_N_ANGLE - 1u);
+            atomicAdd(acc + row[k] + (to >> 1) * kRowStride, to & 1 ? 1u << 16 : 1u);
+            atomicAdd(acc + row[k] + (b >> 1) * kRowStride, b & 1 ? 0u - (1u << 16) : 0u - 1u);
+          }
+        }
+      }
+      if (__any_sync(0xffffffffu, nearest < 2 * kMargin - 1)) {
+        uint32_t amb = 0;
+#pragma unroll
+        for (int k = 0; k < kPerLane; ++k)
+          if (rm[k] >= 0 && ((uint32_t)((int)re - rm[k] + (int)kMargin - 1) & (kTurn - 1u)) < 2 * kMargin - 1)
+            amb |= 1u << k;
+        n_exact += __popc(amb);
+        qn = queue_votes<kCheck>(a, sh, amb, pos, ev0 + q, true, qn);
+      }
+    }
+  }
+  return make_uint2(qn, n_exact);
+}
+
+// A unit of a piece with few events or entries: every vote on its own.  With
+// y' = (x_s - beta_m - margin) << 11 (count_angle), one 32 x 32 -> 64 multiply
+// 15 y' gives the plane in its high word, the half of the counter word in the
+// top bit of its low word and the position inside the bin in the rest: a vote
+// is unambiguous exactly when 2 low is at most kSpan, and the bin is then that
+// of y (y' wraps only for ambiguous votes, to bin 29, so every provisional
+// bin is in [0, 29]).
+template <bool kCheck>
+__device__ __noinline__ uint2 count_unit(const VoteArgs& a, const VoteShared& sh, uint32_t start, uint32_t end,
+                                           uint32_t ev0, uint32_t cnt, uint32_t qn) {
+  uint32_t n_exact = 0;
+  constexpr uint32_t kSpan = (kTurn - 2 * kMargin) << kAngleShift;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t* const entries = a.entries;
+  uint32_t* const acc = smem + kOffAcc;
+  for (uint32_t pos = start; pos < end; pos += kBlock) {
+    const uint32_t n = min((uint32_t)kBlock, end - pos);
+    uint32_t c[kPerLane];
+    load_block(entries, pos, end, c);
+    for (uint32_t g = 0; g < cnt; ++g) {
+      const uint32_t base = count_angle(smem[kOffEvW + ev0 + g], 0u);
+      uint32_t amb = 0;
+#pragma unroll
+      for (int k = 0; k < kPerLane; ++k) {
+        if (32u * k < n && in_range<kCheck>(a, 14, c[k] >> PPF_ANGLE_BITS, kRowStride)) {
+          const unsigned long long p = (unsigned long long)(base - (c[k] << kAngleShift)) * (PPF_N_ANGLE / 2);
+          const uint32_t hi = (uint32_t)(p >> 32), lo = (uint32_t)p;
+          atomicAdd(acc + hi * kRowStride + (c[k] >> PPF_ANGLE_BITS), 1u + (lo >> 31) * 65535u);
+          if ((lo << 1) > kSpan) amb |= 1u << k;
+        }
+      }
+      if (__any_sync(0xffffffffu, amb != 0u)) {
+#pragma unroll
+        for (int k = 0; k < kPerLane; ++k)
+          if (32u * k + lane >= n) amb &= ~(1u << k);
+        n_exact += __popc(amb);
+        qn = queue_votes<kCheck>(a, sh, amb, pos, ev0 + g, false, qn);
+      }
+    }
+  }
+  return make_uint2(qn, n_exact);
+}
+
+// A unit whose votes all take the exact path (a degenerate frame vector of
+// the scene pair or of a pair in the run).
+template <bool kCheck>
+__device__ __noinline__ void exact_unit(const VoteArgs& a, const VoteShared& sh, uint32_t start, uint32_t end,
+                                        uint32_t ev0, uint32_t cnt) {
+  for (uint32_t g = 0; g < cnt; ++g) {
+    const float4 p4 = a.s_pts[smem[kOffEvI + ev0 + g]];
+    FrameYZ fs;
+    fs.r1 = sh.f_r1;
+    fs.r2 = sh.f_r2;
+    const float2 v = frame_point_yz(fs, make_float3(p4.x, p4.y, p4.z));
+    for (uint32_t pos = start + (threadIdx.x & 31); pos < end; pos += 32) {
+      const uint32_t row = __ldg(a.entries + pos) >> PPF_ANGLE_BITS;
+      const uint32_t bin = exact_bin<kCheck>(a, pos, v);
+      if (in_range<kCheck>(a, 6, row, a.chunk)) add_cell(row, bin);
+    }
+  }
+}
+
+// A warp's place in the walk over the scene: its next 32 points and the pairs
+// of its buffer that still await their lookup.
+struct WalkState {
+  uint32_t base = 0, n_near = 0;
+};
+
+// Fills the list with the events of s_r from the warps' places on, until the
+// scene ends (false) or the list is full (true; uniform over the block).
+//
+// Warp w takes points 32 w + lane of every 1024.  With the model's feature
+// table it first looks only at the distance: a pair whose distance row has no
+// run is dropped, the others wait in the warp's buffer until there are 32, so
+// that the angles (three acosf), the table lookup and the frame angle run on
+// full warps.  On the bench's scene 9 of 10 pairs are dropped.  Without the
+// table every pair's feature is hashed.
+template <bool kCheck>
+__device__ __forceinline__ bool walk_scene(const VoteArgs& a, uint32_t sr, bool count, WalkState& ws, VoteShared& sh,
+                                           VoteStats& st) {
+  uint32_t* const slot_key = smem + kOffSlotKey;
+  uint32_t* const slot_cnt = smem + kOffSlotCnt;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t* const near = smem + kOffNear + warp * kNearLen;
+  // (the buffers lie over the pieces, which the list's votes have read)
+  __shared__ uint32_t s_near[kVoteWarps][32];
+  if (ws.n_near && lane < ws.n_near) near[lane] = s_near[warp][lane];
+  for (uint32_t i = tid; i < kSlots; i += kVoteThreads) {
+    slot_key[i] = kNoRun;
+    slot_cnt[i] = 0u;
+  }
+  if (tid == 0) sh.n_ev = sh.n_gr = 0u;
+  block_sync();
+  const float4 p4 = sh.p_r;
+  const float3 pr = make_float3(p4.x, p4.y, p4.z);
+  const float inv_d = 1.0f / a.d_dist;
+  bool full = false;
+  for (;;) {
+    // gather pairs until 32 wait or the scene ends
+    while (ws.n_near < 32 && ws.base < a.n_s) {
+      const uint32_t i = ws.base + tid;
+      bool keep = i < a.n_s && i != sr;
+      if (keep && a.lut) {
+        const float4 q = a.s_pts[i];
+        const float3 d = make_float3(q.x - pr.x, q.y - pr.y, q.z - pr.z);
+        const float len = norm3(d);
+        // rows past the flags are looked up by key
+        keep = !isnan(len);
+        if (len < (float)(kFlagRows - 1) * a.d_dist) {
+          const uint32_t nd = (uint32_t)quant_index(len, a.d_dist, inv_d);
+          keep = sh.rows[nd / 32] >> (nd % 32) & 1u;
+        }
+      }
+      const uint32_t in = __ballot_sync(0xffffffffu, keep);
+      if (keep) near[ws.n_near + __popc(in & ((1u << lane) - 1u))] = i;
+      ws.n_near += __popc(in);
+      ws.base += kVoteThreads;
+    }
+    __syncwarp();
+    const uint32_t n = min(ws.n_near, 32u);
+    if (n == 0) break;
+    if (*(volatile uint32_t*)&sh.n_gr > kGroupLimit) {
+      full = true;
+      break;
+    }
+    // one pair per lane: feature, lookup, frame angle
+    uint32_t run = kNoRun, beta = 0, i = 0;
+    bool exact = false;
+    if (lane < n) {
+      i = near[lane];
+      const float4 pi4 = a.s_pts[i], ni4 = a.s_nrm[i], n4 = sh.n_r;
+      const float3 pi = make_float3(pi4.x, pi4.y, pi4.z), ni = make_float3(ni4.x, ni4.y, ni4.z);
+      const float3 nr = make_float3(n4.x, n4.y, n4.z);
+      const float3 d = make_float3(pi.x - pr.x, pi.y - pr.y, pi.z - pr.z);
+      const float len = norm3(d);
+      uint32_t nd = kLutRows;
+      if (a.lut && len < (float)(kLutRows - 1) * a.d_dist) nd = (uint32_t)quant_index(len, a.d_dist, inv_d);
+      if (nd < kLutRows) {
+        run = __ldg(a.lut + nd * kAngleCombos + pair_angles(nr, ni, d, len));
+      } else {
+        const uint32_t key = feature_key(pair_feature(pr, nr, pi, ni, a.d_dist));
+        if (key != 0u) run = ht_lookup(a.ht_keys, a.ht_runs, a.ht_mask, key);
+      }
+      if (run != kNoRun && in_range<kCheck>(a, 2, run, a.K)) {
+        FrameYZ fs;
+        fs.r1 = sh.f_r1;
+        fs.r2 = sh.f_r2;
+        const float2 v = frame_point_yz(fs, pi);
+        exact = fabsf(v.x) + fabsf(v.y) < 1e-12f || !isfinite(v.x) || !isfinite(v.y) || __ldg(a.run_flags + run);
+        beta = angle21(v);
+      }
+    }
+    __syncwarp();
+    const uint32_t hits = __ballot_sync(0xffffffffu, run != kNoRun);
+    if (hits) {
+      // room for all of them, or none is taken and the pairs stay
+      uint32_t at = 0;
+      if (lane == 0) {
+        at = *(volatile uint32_t*)&sh.n_ev;
+        for (;;) {
+          if (at + __popc(hits) > kEvents) {
+            at = kNoRun;
+            break;
+          }
+          const uint32_t was = atomicCAS(&sh.n_ev, at, at + __popc(hits));
+          if (was == at) break;
+          at = was;
+        }
+      }
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at == kNoRun) {
+        full = true;
+        break;
+      }
+      if (run != kNoRun) {
+        at += __popc(hits & ((1u << lane) - 1u));
+        if (count) {
+          st.votes += __ldg(a.run_count + run);
+          st.matched += 1;
+        }
+        // the event's slot and its rank in the group
+        const uint32_t group = run | (exact ? kExactGroup : 0u);
+        uint32_t slot = (group * 0x9E3779B1u) >> 21;
+        for (uint32_t probe = 0; probe < kSlots; ++probe) {
+          uint32_t k = *(volatile uint32_t*)(slot_key + slot);
+          if (k == kNoRun) {
+            k = atomicCAS(slot_key + slot, kNoRun, group);
+            if (k == kNoRun) {
+              atomicAdd(&sh.n_gr, 1u);
+              break;
+            }
+          }
+          if (k == group) break;
+          slot = (slot + 1) & (kSlots - 1);
+        }
+        const uint32_t rank = atomicAdd(slot_cnt + slot, 1u);
+        if (in_range<kCheck>(a, 15, at, kEvents)) {
+          smem[kOffEvW + at] = ((beta + (kTurn >> 1)) & (kTurn - 1u)) * PPF_N_ANGLE;
+          smem[kOffEvI + at] = i;
+          smem[kOffEvK + at] = slot << 16 | rank;
+        }
+      }
+    }
+    // the buffer's rest (at most 31 pairs) moves to its front
+    __syncwarp();
+    const uint32_t rest = ws.n_near - n;
+    const uint32_t moved = lane < rest ? near[n + lane] : 0u;
+    __syncwarp();
+    if (lane < rest) near[lane] = moved;
+    ws.n_near = rest;
+    __syncwarp();
+  }
+  // what waits is kept aside while the list's pieces take the buffers' place
+  // (at most 32 + 31 pairs; those past 32 are walked again)
+  __syncwarp();
+  if (ws.n_near > 32) {
+    // the last step's points start over: nothing of them was looked up
+    const uint32_t first = ws.base - kVoteThreads;
+    ws.n_near = __popc(__ballot_sync(0xffffffffu, near[lane] < first + warp * 32));
+    ws.base = first;
+  }
+  if (lane < ws.n_near) s_near[warp][lane] = near[lane];
+  __syncwarp();
+  return __syncthreads_or(full);
+}
+
+// Sorts a swept piece's events by R (rank by comparison: at most 255 events)
+// and returns an upper bound of how many of them one entry can vote into one
+// bin: its votes for a bin come from one bin's width of event angles, plus
+// the margin on both sides for votes near an edge, which lies within four
+// neighbouring half bins.
+__device__ __forceinline__ uint32_t sort_piece(uint32_t ev0, uint32_t cnt) {
+  uint32_t* const tab = warp_tab();
+  const uint32_t lane = threadIdx.x & 31;
+  constexpr int kPer = (kPieceEvents + 31) / 32;
+  uint32_t* const ew = smem + kOffEvW + ev0;
+  uint32_t* const ei = smem + kOffEvI + ev0;
+  uint32_t w[kPer], pi[kPer], rank[kPer];
+  constexpr uint32_t kHalves = 2 * PPF_N_ANGLE;
+  static_assert(kHalves <= kTabWords, "a counter per half bin");
+  for (uint32_t k = lane; k < kHalves; k += 32) tab[k] = 0u;
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < kPer; ++m) {
+    const uint32_t j = 32u * m + lane;
+    w[m] = j < cnt ? ew[j] : 0u;
+    pi[m] = j < cnt ? ei[j] : 0u;
+    rank[m] = 0;
+    if (j < cnt) atomicAdd(tab + (w[m] >> (PPF_ANGLE_BITS - 1)), 1u);
+  }
+  for (uint32_t q = 0; q < cnt; ++q) {
+    const uint32_t r = ew[q] & (kTurn - 1u);
+#pragma unroll
+    for (int m = 0; m < kPer; ++m) {
+      if (32u * m < cnt) {
+        const uint32_t own = w[m] & (kTurn - 1u);
+        rank[m] += (r < own || (r == own && q < 32u * m + lane)) ? 1u : 0u;
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < kPer; ++m) {
+    if (32u * m + lane < cnt) {
+      ew[rank[m]] = w[m];
+      ei[rank[m]] = pi[m];
+    }
+  }
+  uint32_t win = 0;
+  for (uint32_t k = lane; k < kHalves; k += 32) {
+    uint32_t four = 0;
+    for (uint32_t o = k; o < k + 4; ++o) four += tab[o >= kHalves ? o - kHalves : o];
+    win = max(win, four);
+  }
+  win = __reduce_max_sync(0xffffffffu, win);
+  __syncwarp();
+  return win;
+}
+
+// Groups the list's events by run (counting sort through registers, in
+// place), cuts the groups into pieces and sorts the swept ones.  Returns the
+// number of pieces.
+template <bool kCheck>
+__device__ __forceinline__ uint32_t group_events(const VoteArgs& a, uint32_t n_ev, VoteShared& sh) {
+  uint32_t* const slot_key = smem + kOffSlotKey;
+  uint32_t* const slot_cnt = smem + kOffSlotCnt;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  const uint32_t key0 = slot_key[2 * tid], key1 = slot_key[2 * tid + 1];
+  const uint32_t c0 = slot_cnt[2 * tid], c1 = slot_cnt[2 * tid + 1];
+  const uint32_t n0 = (c0 + kPieceEvents - 1) / kPieceEvents, n1 = (c1 + kPieceEvents - 1) / kPieceEvents;
+  uint2 total;
+  const uint2 at = block_excl_scan(make_uint2(c0 + c1, n0 + n1), sh.scan2, total);
+  uint32_t w[kEventsPerThread], ei[kEventsPerThread], ek[kEventsPerThread];
+#pragma unroll
+  for (uint32_t k = 0; k < kEventsPerThread; ++k) {
+    const uint32_t j = tid + k * kVoteThreads;
+    w[k] = ei[k] = ek[k] = 0;
+    if (j < n_ev) {
+      w[k] = smem[kOffEvW + j];
+      ei[k] = smem[kOffEvI + j];
+      ek[k] = smem[kOffEvK + j];
+    }
+  }
+  slot_cnt[2 * tid] = at.x;
+  slot_cnt[2 * tid + 1] = at.x + c0;
+  uint32_t p = at.y;
+  for (uint32_t o = 0; o < c0 && in_range<kCheck>(a, 24, p, kMaxPieces); o += kPieceEvents, ++p) {
+    smem[kOffPcRun + p] = key0 & ~kExactGroup;
+    const uint32_t n = min(kPieceEvents, c0 - o);
+    smem[kOffPcInf + p] = piece_info(at.x + o, n, key0 & kExactGroup, n);
+  }
+  for (uint32_t o = 0; o < c1 && in_range<kCheck>(a, 24, p, kMaxPieces); o += kPieceEvents, ++p) {
+    smem[kOffPcRun + p] = key1 & ~kExactGroup;
+    const uint32_t n = min(kPieceEvents, c1 - o);
+    smem[kOffPcInf + p] = piece_info(at.x + c0 + o, n, key1 & kExactGroup, n);
+  }
+  block_sync();  // offsets visible, every event in a register
+#pragma unroll
+  for (uint32_t k = 0; k < kEventsPerThread; ++k) {
+    if (tid + k * kVoteThreads < n_ev) {
+      const uint32_t to = slot_cnt[ek[k] >> 16] + (ek[k] & 0xffffu);
+      if (in_range<kCheck>(a, 25, to, n_ev)) {
+        smem[kOffEvW + to] = w[k];
+        smem[kOffEvI + to] = ei[k];
+      }
+    }
+  }
+  block_sync();  // the slots are free for the tables from here on
+  for (uint32_t q = warp; q < total.y; q += kVoteWarps) {
+    const uint32_t inf = smem[kOffPcInf + q];
+    const uint32_t ev0 = inf & 0x1fffu, cnt = (inf >> 13) & 0xffu;
+    if (cnt < kSweepMin || (inf >> 21 & 1u)) continue;
+    const uint32_t win = sort_piece(ev0, cnt);
+    if ((tid & 31) == 0) smem[kOffPcInf + q] = piece_info(ev0, cnt, false, win);
+  }
+  block_sync();
+  return total.y;
+}
+
+// Adds the accumulator's 16-bit counters to the block's 32-bit counters in
+// global memory and clears them (each thread always handles the same rows).
+__device__ __forceinline__ void spill_acc(const VoteArgs& a, bool first) {
+  uint32_t* const acc = smem + kOffAcc;
+  uint2* const sp = a.spill + (size_t)blockIdx.x * kSpillWords;
+  block_sync();
+  for (uint32_t row = threadIdx.x; row < a.chunk; row += kVoteThreads) {
+#pragma unroll
+    for (uint32_t j = 0; j < kPlanes; ++j) {
+      const uint32_t v = acc[j * kRowStride + row];
+      uint2* const at = sp + j * kRowStride + row;
+      uint2 s = make_uint2(0u, 0u);
+      if (!first) s = *at;
+      *at = make_uint2(s.x + (v & 0xffffu), s.y + (v >> 16));
+      acc[j * kRowStride + row] = 0u;
+    }
+  }
+  block_sync();
+}
+
+// The units [u0, u1) of the current chunk, events [s0, s1) of each piece.
+template <bool kCheck>
+__device__ __forceinline__ void vote_units(const VoteArgs& a, VoteShared& sh, VoteStats& st, uint32_t n_pieces,
+                                           uint32_t u0, uint32_t u1, uint32_t s0, uint32_t s1, uint32_t shift,
+                                           uint32_t item) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t* const pc_unit = smem + kOffPcUnit;
+  if (tid == 0) sh.next = u0 + kVoteWarps;
+  block_sync();
+  uint32_t qn = 0;
+  const uint32_t stride = (n_pieces + 31) / 32;
+  uint32_t u = u0 + warp;
+  while (u < u1) {
+    // piece p with pc_unit[p] <= u < pc_unit[p + 1] (pc_unit is
+    // nondecreasing): one ballot over every stride-th piece, then over the
+    // stride (at most 49) pieces behind it
+    const uint32_t blk =
+        31u - __clz(__ballot_sync(0xffffffffu, lane * stride <= n_pieces && pc_unit[min(lane * stride, n_pieces)] <= u));
+    uint32_t p = blk * stride;
+    uint32_t in = 0;
+    for (uint32_t o = 1; o < stride; o += 32)
+      in += __popc(__ballot_sync(0xffffffffu, o + lane < stride && p + o + lane <= n_pieces &&
+                                                  pc_unit[min(p + o + lane, n_pieces)] <= u));
+    p += in;
+    const uint32_t inf = smem[kOffPcInf + min(p, n_pieces - 1)];
+    const uint32_t lo = smem[kOffPcLo + p], len = smem[kOffPcLen + p];
+    const uint32_t skip = (u - pc_unit[p]) << shift;
+    const uint32_t start = lo + skip;
+    uint32_t end = lo + min(len, skip + (1u << shift));
+    // Always-on guard (one compare per unit): a unit outside its sub-run or
+    // the entry array is recorded, raises kFlagBadIndex and is skipped, so
+    // the lookup fails instead of the kernel reading outside the entries.
+    if (p >= n_pieces || skip >= len || end > a.P || start >= end) {
+      if (lane == 0) {
+        if (atomicCAS(&a.bad[3], 0ull, 1ull) == 0ull) {
+          a.bad[4] = ((unsigned long long)p << 32) | u;
+          a.bad[5] = ((unsigned long long)n_pieces << 32) | pc_unit[min(p, n_pieces)];
+          a.bad[6] = ((unsigned long long)lo << 32) | len;
+          a.bad[7] = ((unsigned long long)u0 << 32) | u1;
+          a.bad[8] = ((unsigned long long)s0 << 32) | item;
+          a.bad[9] = ((unsigned long long)warp << 32) | inf;
+        }
+        atomicOr(a.flags, (uint32_t)kFlagBadIndex);
+      }
+      end = start;
+    }
+    const uint32_t cnt = (inf >> 13) & 0xffu;
+    const uint32_t ev0 = (inf & 0x1fffu) + min(s0, cnt), n_ev = min(s1, cnt) - min(s0, cnt);
+    if (end > start && n_ev) {
+      if (inf >> 21 & 1u) {
+        exact_unit<kCheck>(a, sh, start, end, ev0, n_ev);
+        if (lane == 0) st.exact += (unsigned long long)(end - start) * n_ev;
+      } else {
+        const uint2 r = sweep_pays(cnt, len) ? sweep_unit<kCheck>(a, sh, start, end, ev0, n_ev, qn)
+                                         : count_unit<kCheck>(a, sh, start, end, ev0, n_ev, qn);
+        qn = r.x;
+        st.exact += r.y;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) u = atomicAdd(&sh.next, 1u);
+    u = __shfl_sync(0xffffffffu, u, 0);
+  }
+  if (qn) drain_queue<kCheck>(a, sh, qn);
+  block_sync();
+}
+
+// Largest 16-bit counter of the accumulator.
+__device__ __forceinline__ uint32_t acc_max(const VoteArgs& a, VoteShared& sh) {
+  uint32_t m = 0;
+  for (uint32_t row = threadIdx.x; row < a.chunk; row += kVoteThreads) {
+#pragma unroll
+    for (uint32_t j = 0; j < kPlanes; ++j) {
+      const uint32_t v = smem[kOffAcc + j * kRowStride + row];
+      m = max(m, max(v & 0xffffu, v >> 16));
+    }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) sh.wmax[threadIdx.x >> 5] = m;
+  block_sync();
+  m = __reduce_max_sync(0xffffffffu, sh.wmax[threadIdx.x & 31]);
+  block_sync();
+  return m;
+}
+
+// Votes of the grouped events into chunk c.  `bound` is the largest value a
+// 16-bit counter can hold so far.  Pieces that could take one past 65535 go in
+// batches; between two the bound is replaced by the largest counter, and the
+// accumulator spilled when that is past half the range.
+template <bool kCheck>
+__device__ __forceinline__ void vote_chunk(const VoteArgs& a, uint32_t c, uint32_t n_pieces, VoteShared& sh,
+                                           VoteStats& st, uint32_t& bound, bool& spilled, uint32_t item) {
+  if (n_pieces == 0) return;
+  const uint32_t tid = threadIdx.x;
+  uint32_t shift = a.unit_shift;
+  uint32_t lo[2], len[2], units[2], inc[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t p = 2 * tid + k;
+    lo[k] = len[k] = units[k] = inc[k] = 0;
+    if (p < n_pieces) {
+      const uint32_t run = smem[kOffPcRun + p], win = smem[kOffPcInf + p] >> 22;
+      if (in_range<kCheck>(a, 16, run, a.K)) {
+        const uint32_t* sp = a.split + (size_t)run * (a.n_chunks + 1) + c;
+        lo[k] = __ldg(sp);
+        len[k] = __ldg(sp + 1) - lo[k];
+        if (kCheck && !in_range<kCheck>(a, 3, (unsigned long long)lo[k] + len[k], a.P + 1)) len[k] = 0;
+        // win <= 256 events, at most run_maxl <= 65535 entries each
+        inc[k] = len[k] ? min(win * __ldg(a.run_maxl + run), kCounterMax + 1u) : 0u;
+      }
+    }
+  }
+  uint2 total, at;
+  for (;;) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) units[k] = (len[k] >> shift) + (len[k] & ((1u << shift) - 1u) ? 1u : 0u);
+    at = block_excl_scan(make_uint2(units[0] + units[1], inc[0] + inc[1]), sh.scan2, total);
+    // few units leave warps idle at the end of the phase: halve them
+    if (total.x >= kMinUnits || shift <= kMinUnitShift) break;
+    --shift;
+    block_sync();
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t p = 2 * tid + k;
+    if (p <= n_pieces) {
+      smem[kOffPcLo + p] = lo[k];
+      smem[kOffPcLen + p] = len[k];
+      smem[kOffPcUnit + p] = at.x + (k ? units[0] : 0u);
+      smem[kOffPcInc + p] = at.y + (k ? inc[0] : 0u);
+    }
+  }
+  block_sync();
+  if (total.x == 0) return;
+  auto spill = [&]() {
+    if (!bound) return;
+    spill_acc(a, !spilled);
+    spilled = true;
+    bound = 0;
+  };
+  const uint32_t* const pc_inc = smem + kOffPcInc;
+  const uint32_t* const pc_unit = smem + kOffPcUnit;
+  for (uint32_t p0 = 0; p0 < n_pieces;) {
+    if (bound && bound + (total.y - pc_inc[p0]) > kCounterMax) {
+      bound = acc_max(a, sh);
+      if (bound > kCounterMax / 2) spill();
+    }
+    uint32_t p1 = p0, hi = n_pieces;  // the last p1 whose pieces from p0 on fit
+    while (p1 < hi) {
+      const uint32_t mid = (p1 + hi + 1) / 2;
+      if (bound + (pc_inc[mid] - pc_inc[p0]) <= kCounterMax) p1 = mid;
+      else hi = mid - 1;
+    }
+    if (p1 > p0) {
+      vote_units<kCheck>(a, sh, st, n_pieces, pc_unit[p0], pc_unit[p1], 0, kPieceEvents, shift, item);
+      bound += pc_inc[p1] - pc_inc[p0];
+      p0 = p1;
+    } else if (bound) {
+      spill();  // and try the piece again with all the range
+    } else {
+      // one piece alone: as many of its events at a time as surely fit
+      const uint32_t sub = max(1u, kCounterMax / max(1u, __ldg(a.run_maxl + smem[kOffPcRun + p0])));
+      const uint32_t cnt = (smem[kOffPcInf + p0] >> 13) & 0xffu;
+      for (uint32_t s0 = 0; s0 < cnt; s0 += sub) {
+        spill();
+        vote_units<kCheck>(a, sh, st, n_pieces, pc_unit[p0], pc_unit[p0 + 1], s0, min(s0 + sub, cnt), shift, item);
+        bound = kCounterMax;
+      }
+      ++p0;
+    }
+  }
+}
+
+// Running maximum and emission of the accumulator's cells.
+template <bool kCheck>
+__device__ __forceinline__ void emit_chunk(const VoteArgs& a, uint32_t sr, uint32_t c, uint32_t item, bool spilled,
+                                           VoteShared& sh) {
+  const uint32_t* const acc = smem + kOffAcc;
+  const uint2* const sp = a.spill + (size_t)blockIdx.x * kSpillWords;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // calls f(row, bin, count) for this thread's counters (its own rows)
+  auto each = [&](auto f) {
+    for (uint32_t row = tid; row < a.chunk; row += kVoteThreads) {
+#pragma unroll
+      for (uint32_t j = 0; j < kPlanes; ++j) {
+        const uint32_t v = acc[j * kRowStride + row];
+        uint2 n = make_uint2(v & 0xffffu, v >> 16);
+        if (spilled) n = sp[j * kRowStride + row];
+        f(row, 2 * j, n.x);
+        f(row, 2 * j + 1, n.y);
+      }
+      f(row, (uint32_t)PPF_N_ANGLE, acc[kPlanes * kRowStride + row]);
+    }
+  };
+  uint32_t lmax = 0;
+  each([&](uint32_t, uint32_t, uint32_t cnt) { lmax = max(lmax, cnt); });
+  lmax = __reduce_max_sync(0xffffffffu, lmax);
+  if (lane == 0) sh.wmax[warp] = lmax;
+  block_sync();
+  if (warp == 0) {
+    const uint32_t m = __reduce_max_sync(0xffffffffu, sh.wmax[lane]);
+    if (lane == 0) sh.max = max(atomicMax(a.global_max, m), m);
+  }
+  block_sync();
+  const float floor_v = a.floor >= 0.f ? a.floor : a.thr * (float)sh.max;
+  auto kept = [&](uint32_t cnt) { return cnt != 0u && (a.emit_all || (float)cnt > floor_v); };
+  // All-or-nothing slot reservation for the chunk's cells: a chunk that does
+  // not fit writes nothing and is queued for a second launch after the
+  // buffer has grown, so the buffer never holds a partial chunk.
+  uint32_t my_n = 0;
+  each([&](uint32_t, uint32_t, uint32_t cnt) { my_n += kept(cnt) ? 1u : 0u; });
+  uint32_t item_total;
+  const uint32_t my_off = block_excl_scan(my_n, sh.scan_emit, item_total);
+  if (item_total == 0) return;  // uniform
+  if (warp == 0) {
+    // The whole warp walks the reservation loop in lockstep (lane 0 issues
+    // the atomics, every exit condition is warp-uniform).
+    uint32_t base_slot = 0xffffffffu;
+    if (lane == 0) atomicAdd(a.n_needed, (unsigned long long)item_total);
+    uint32_t old = 0;
+    if (lane == 0) old = *(volatile uint32_t*)a.n_cand;
+    old = __shfl_sync(0xffffffffu, old, 0);
+    for (int tries = 0; tries < (1 << 20); ++tries) {
+      if ((unsigned long long)old + item_total > a.cand_cap) break;
+      uint32_t prev = 0;
+      if (lane == 0) prev = atomicCAS(a.n_cand, old, old + item_total);
+      prev = __shfl_sync(0xffffffffu, prev, 0);
+      if (prev == old) {
+        base_slot = old;
+        break;
+      }
+      old = prev;
+    }
+    if (base_slot == 0xffffffffu && lane == 0) {
+      const uint32_t k = atomicAdd(a.n_redo, 1u);
+      if (in_range<kCheck>(a, 9, k, a.n_items_total)) a.redo_items[k] = item;
+    }
+    if (lane == 0) sh.base = base_slot;
+  }
+  block_sync();
+  const uint32_t item_base = sh.base;
+  if (item_base == 0xffffffffu) return;
+  uint32_t slot = item_base + my_off;
+  each([&](uint32_t row, uint32_t bin, uint32_t cnt) {
+    if (!kept(cnt)) return;
+    const uint32_t mr = c * a.chunk + row;
+    if (in_range<kCheck>(a, 10, slot, a.cand_cap)) {
+      a.cand_code[slot] = ((unsigned long long)sr << 32) | ((unsigned long long)mr << 6) | bin;
+      a.cand_count[slot] = cnt;
+    }
+    ++slot;
+  });
+}
+
+// One work item of request `a` (slot_of_item indexes a's items, or
+// a.item_list).  Called by every thread of the block.  A scene whose matched
+// pairs fit the list is walked once for all chunks of the item; otherwise
+// every chunk walks it again in as many parts as it takes.
+template <bool kCheck>
+__device__ __forceinline__ void vote_item(const VoteArgs& a, uint32_t slot_of_item, VoteShared& sh, VoteStats& st) {
+  const uint32_t tid = threadIdx.x;
+  uint32_t rq, c0, c1;
+  if (a.item_list) {
+    const uint32_t item = a.item_list[slot_of_item];
+    rq = item / a.n_chunks;
+    c0 = item - rq * a.n_chunks;
+    c1 = c0 + 1;
+  } else {
+    rq = slot_of_item / a.n_cg;
+    c0 = (slot_of_item - rq * a.n_cg) * a.cpi;
+    c1 = min(a.n_chunks, c0 + a.cpi);
+  }
+  // ref < n_ref, so sr = ref * ref_df < n_s
+  const uint32_t ref = (uint32_t)(((unsigned long long)rq * a.perm_mul) % a.n_ref);
+  const uint32_t sr = ref * a.ref_df;
+  // thread 0 publishes the frame of s_r, warp 1 the model's row flags; the
+  // barrier at the start of the walk makes them visible, and the previous item's readers are past the item-fetch
+  // barrier before it is overwritten
+  if (tid == 0) {
+    const float4 p4 = a.s_pts[sr], n4 = a.s_nrm[sr];
+    const FrameYZ f = frame_yz(make_float3(p4.x, p4.y, p4.z), make_float3(n4.x, n4.y, n4.z));
+    sh.p_r = p4;
+    sh.n_r = n4;
+    sh.f_r1 = f.r1;
+    sh.f_r2 = f.r2;
+  }
+  static_assert(kFlagRows / 32 == 32, "a row flag word per lane");
+  if (tid >= 32 && tid < 64 && a.lut) sh.rows[tid - 32] = __ldg(a.row_flags + tid - 32);
+  bool whole = false;  // the list holds all events of s_r
+  uint32_t n_pieces = 0;
+  for (uint32_t c = c0; c < c1; ++c) {
+    const uint32_t item = rq * a.n_chunks + c;
+    if (c > c0) block_sync();  // the previous chunk's emission has read the accumulator
+    for (uint32_t row = tid; row < a.chunk; row += kVoteThreads) {
+#pragma unroll
+      for (uint32_t j = 0; j <= kPlanes; ++j) smem[kOffAcc + j * kRowStride + row] = 0u;
+    }
+    uint32_t bound = 0;
+    bool spilled = false;
+    if (whole) {
+      vote_chunk<kCheck>(a, c, n_pieces, sh, st, bound, spilled, item);
+    } else {
+      const bool count = c == 0 && !a.item_list;
+      WalkState w;
+      for (bool first = true;; first = false) {
+        const bool more = walk_scene<kCheck>(a, sr, count, w, sh, st);
+        const uint32_t n_ev = sh.n_ev;
+        n_pieces = n_ev ? group_events<kCheck>(a, n_ev, sh) : 0;
+        whole = first && !more;
+        vote_chunk<kCheck>(a, c, n_pieces, sh, st, bound, spilled, item);
+        if (!more) break;
+        block_sync();  // the votes' reads of the list are over
+      }
+    }
+    block_sync();  // all votes of the chunk are counted
+    if (spilled && bound) spill_acc(a, false);
+    emit_chunk<kCheck>(a, sr, c, item, spilled, sh);
+  }
+  // The item-fetch barrier of the caller separates these reads of the
+  // accumulator from the next item's clear.
+}
+
+template <bool kCheck>
+__global__ void __launch_bounds__(kVoteThreads, 1) vote_kernel(const __grid_constant__ VoteArgs a) {
   __shared__ VoteShared sh;
   VoteStats st;
   for (;;) {
@@ -605,6 +1346,18 @@ uint32_t gcd_u32(uint32_t x, uint32_t y) {
   return x;
 }
 
+// Chunks per work item.  One item per scene reference point walks the scene
+// once for all chunks; with few reference points the chunks are shared out
+// until there are about 16 items per SM (8 / 16 / 32: 71.8 / 69.0 / 69.5 ms over
+// the bench's four models at ref_point_df 50).
+void set_items(VoteArgs& a, size_t refs_in_launch) {
+  const size_t want = 16 * (size_t)sm_count();
+  size_t split = refs_in_launch ? (want + refs_in_launch - 1) / refs_in_launch : 1;
+  split = std::min<size_t>(std::max<size_t>(split, 1), a.n_chunks);
+  a.cpi = (uint32_t)((a.n_chunks + split - 1) / split);
+  a.n_cg = (a.n_chunks + a.cpi - 1) / a.cpi;
+}
+
 VoteArgs make_args(const Model& m, const SceneData& s) {
   const ModelTables& t = m.t;
   VoteArgs a{};
@@ -624,8 +1377,15 @@ VoteArgs make_args(const Model& m, const SceneData& s) {
   a.n_m = t.n;
   a.chunk = t.chunk;
   a.n_chunks = t.n_chunks;
-  const uint32_t shift = m.seg_shift.load(std::memory_order_relaxed);
-  a.seg_shift = shift ? shift : kSegShiftDefault;
+  a.run_maxl = t.run_maxl.as<uint32_t>();
+  if (t.lut_quantum > 0.f && t.lut_quantum == s.d_dist) {
+    a.lut = t.lut.as<uint32_t>();
+    a.row_flags = t.row_flags.as<uint32_t>();
+  }
+  a.r_shift = t.r_shift;
+  // a unit of the vote phase is a quarter of a segment, at least one block
+  const uint32_t segment = vote_segment_shift(*m.ctx);
+  a.unit_shift = segment < 9 ? 7 : segment - 2;
   a.s_pts = s.pts.as<float4>();
   a.s_nrm = s.nrm.as<float4>();
   a.n_s = s.n;
@@ -643,13 +1403,29 @@ VoteArgs make_args(const Model& m, const SceneData& s) {
 
 }  // namespace
 
+void init_vote_kernels(int smem_limit) {
+  PPF_REQUIRE((size_t)smem_limit >= kVoteSmemBytes, PPF_ERR_CUDA, "vote accumulator too large for this device");
+  auto set = [&](auto kernel) {
+    PPF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVoteSmemBytes));
+  };
+  set(vote_kernel<false>);
+  set(vote_kernel<true>);
+  set(vote_batch_kernel<false>);
+  set(vote_batch_kernel<true>);
+}
+
+void reserve_vote_spill(Context& ctx) { ctx.vote_spill.reserve(sm_count() * kSpillWords * sizeof(uint2)); }
+
 VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit_all, float floor) {
   VoteResult r;
   cudaStream_t stream = ctx.stream;
   VoteArgs a = make_args(m, s);
   a.emit_all = emit_all ? 1 : 0;
   a.floor = floor;
-  const uint32_t n_items = a.n_ref * a.n_chunks;
+  set_items(a, a.n_ref);
+  reserve_vote_spill(ctx);
+  a.spill = ctx.vote_spill.as<uint2>();
+  const uint32_t n_items = a.n_ref * a.n_cg;
   if (s.n < 2 || n_items == 0) return r;
   // counters: [0] work, [1] max, [2] n_cand, [3] n_redo, [4..9] 3 x u64 stats,
   // [10..11] u64 n_needed, [12] work counter of the second launch
@@ -667,23 +1443,20 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
   a.flags = ctx.flags.as<uint32_t>();
   ctx.cand_codes.reserve(ctx.cand_cap * sizeof(unsigned long long));
   ctx.cand_counts.reserve(ctx.cand_cap * sizeof(uint32_t));
-  ctx.redo_items.reserve((size_t)n_items * sizeof(uint32_t));
+  ctx.redo_items.reserve((size_t)a.n_ref * a.n_chunks * sizeof(uint32_t));
   a.cand_code = ctx.cand_codes.as<unsigned long long>();
   a.cand_count = ctx.cand_counts.as<uint32_t>();
   a.cand_cap = (uint32_t)std::min<size_t>(ctx.cand_cap, 0xffffffffu);
   a.redo_items = ctx.redo_items.as<uint32_t>();
   a.item_list = nullptr;
   a.n_items = n_items;
-  a.n_items_total = n_items;
+  a.n_items_total = a.n_ref * a.n_chunks;
   const bool check = ctx.checks;
   a.bad = reinterpret_cast<unsigned long long*>(ctx.flags.as<uint32_t>() + 8);
   auto kernel = check ? vote_kernel<true> : vote_kernel<false>;
 
-  const size_t smem = kVoteQueueBytes + vote_acc_words(a.chunk) * 4;
-  PPF_REQUIRE((int)smem <= ctx.vote_smem_limit, PPF_ERR_INTERNAL, "vote accumulator too large");
-  PPF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   PPF_CUDA(cudaEventRecord(ctx.ev[0], stream));
-  kernel<<<(unsigned)std::min<size_t>(n_items, (size_t)sm_count()), kVoteThreads, smem, stream>>>(a);
+  kernel<<<(unsigned)std::min<size_t>(n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
   PPF_CUDA(cudaGetLastError());
   ctx.launches++;
   uint32_t h[16];
@@ -714,7 +1487,7 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
     a.n_items = h[3];
     a.work_counter = cnt + 12;
     PPF_CUDA(cudaMemsetAsync(a.n_redo, 0, 4, stream));
-    kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, smem, stream>>>(a);
+    kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
     r.n_redo = h[3];
@@ -764,20 +1537,26 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
   PPF_CUDA(cudaMemsetAsync(ctx.batch_counters.ptr, 0, (n + 1) * 64, stream));
   PPF_CUDA(cudaMemsetAsync(ctx.flags.ptr, 0, 32 + 80, stream));
   uint32_t* cnt0 = ctx.batch_counters.as<uint32_t>();
-  size_t total = 0, smem = kVoteQueueBytes;
+  size_t total = 0, refs = 0;
+  std::vector<size_t> redo_off(n + 1, 0);
   for (size_t i = 0; i < n; ++i) {
-    const VoteArgs a0 = make_args(*reqs[i].m, *reqs[i].s);
-    const uint64_t items = reqs[i].s->n < 2 ? 0 : (uint64_t)a0.n_ref * a0.n_chunks;
-    total += items;
-    PPF_REQUIRE(total < 0xffffffffull, PPF_ERR_INVALID_ARGUMENT, "more than 2^32 work items in one batch");
-    item_off[i + 1] = (uint32_t)total;
-    smem = std::max(smem, kVoteQueueBytes + vote_acc_words(a0.chunk) * 4);
+    args[i] = make_args(*reqs[i].m, *reqs[i].s);
+    if (reqs[i].s->n >= 2) refs += args[i].n_ref;
   }
-  PPF_REQUIRE((int)smem <= ctx.vote_smem_limit, PPF_ERR_INTERNAL, "vote accumulator too large");
-  ctx.batch_redo.reserve(std::max<size_t>(total, 1) * sizeof(uint32_t));
+  for (size_t i = 0; i < n; ++i) {
+    set_items(args[i], refs);
+    const bool any = reqs[i].s->n >= 2;
+    total += any ? (uint64_t)args[i].n_ref * args[i].n_cg : 0;
+    redo_off[i + 1] = redo_off[i] + (any ? (uint64_t)args[i].n_ref * args[i].n_chunks : 0);
+    PPF_REQUIRE(redo_off[i + 1] < 0xffffffffull, PPF_ERR_INVALID_ARGUMENT,
+                "more than 2^32 work items in one batch");
+    item_off[i + 1] = (uint32_t)total;
+  }
+  ctx.batch_redo.reserve(std::max<size_t>(redo_off[n], 1) * sizeof(uint32_t));
+  reserve_vote_spill(ctx);
   for (size_t i = 0; i < n; ++i) {
     VoteArgs& a = args[i];
-    a = make_args(*reqs[i].m, *reqs[i].s);
+    a.spill = ctx.vote_spill.as<uint2>();
     a.emit_all = 0;
     a.floor = -1.f;
     uint32_t* cnt = cnt0 + 16 * i;
@@ -796,10 +1575,10 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
     a.cand_code = reqs[i].codes.as<unsigned long long>();
     a.cand_count = reqs[i].counts.as<uint32_t>();
     a.cand_cap = (uint32_t)reqs[i].cap;
-    a.redo_items = ctx.batch_redo.as<uint32_t>() + item_off[i];
+    a.redo_items = ctx.batch_redo.as<uint32_t>() + redo_off[i];
     a.item_list = nullptr;
     a.n_items = item_off[i + 1] - item_off[i];
-    a.n_items_total = a.n_items;
+    a.n_items_total = (uint32_t)(redo_off[i + 1] - redo_off[i]);
   }
   ctx.batch_args.reserve(n * sizeof(VoteArgs));
   ctx.batch_off.reserve((n + 1) * sizeof(uint32_t));
@@ -817,8 +1596,7 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
   auto kernel = check ? vote_kernel<true> : vote_kernel<false>;
   PPF_CUDA(cudaEventRecord(ctx.ev[0], stream));
   if (total) {
-    PPF_CUDA(cudaFuncSetAttribute(bkernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    bkernel<<<(unsigned)std::min<size_t>(total, (size_t)sm_count()), kVoteThreads, smem, stream>>>(b);
+    bkernel<<<(unsigned)std::min<size_t>(total, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(b);
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
   }
@@ -854,9 +1632,7 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
     a.n_items = hc[3];
     a.work_counter = cnt0 + 16 * i + 12;
     PPF_CUDA(cudaMemsetAsync(a.n_redo, 0, 4, stream));
-    const size_t smem_i = kVoteQueueBytes + vote_acc_words(a.chunk) * 4;
-    PPF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
-    kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, smem_i, stream>>>(a);
+    kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
     PPF_CUDA(cudaMemcpyAsync(hc, cnt0 + 16 * i, 64, cudaMemcpyDeviceToHost, stream));
@@ -890,84 +1666,6 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
   }
 }
 
-void tune_vote_segments(Context& ctx, Model& m, const SceneData& s, uint64_t signature) {
-  if (m.seg_shift) return;
-  if (ctx.forced_seg_shift) {
-    m.seg_shift = ctx.forced_seg_shift;
-    return;
-  }
-  auto it = ctx.seg_tuned.find(signature);
-  if (it != ctx.seg_tuned.end()) {
-    m.seg_shift = it->second;
-    return;
-  }
-  if (!ctx.tune || s.n < 2) {
-    m.seg_shift = kSegShiftDefault;
-    return;
-  }
-  cudaStream_t stream = ctx.stream;
-  VoteArgs a = make_args(m, s);
-  const uint32_t n_items = a.n_ref * a.n_chunks;
-  // about two items per SM: the first items of the pass's scrambled order of
-  // scene reference points, for every chunk of the model
-  const uint32_t sample = std::min<uint32_t>(n_items, 2u * (uint32_t)sm_count());
-  // The sample launches count and emit nothing: no cell exceeds an infinite
-  // floor.  Their counters live in a buffer of their own.
-  ctx.tune_counters.reserve(64 + 32 + 80);
-  uint32_t* cnt = ctx.tune_counters.as<uint32_t>();
-  a.emit_all = 0;
-  a.floor = INFINITY;
-  a.work_counter = cnt + 0;
-  a.global_max = cnt + 1;
-  a.n_cand = cnt + 2;
-  a.n_redo = cnt + 3;
-  a.stats = reinterpret_cast<unsigned long long*>(cnt + 4);
-  a.n_needed = reinterpret_cast<unsigned long long*>(cnt + 10);
-  a.flags = cnt + 16;
-  a.bad = reinterpret_cast<unsigned long long*>(cnt + 24);
-  a.cand_code = nullptr;
-  a.cand_count = nullptr;
-  a.cand_cap = 0;
-  a.redo_items = nullptr;
-  a.n_items_total = 0;
-  a.item_list = nullptr;
-  a.n_items = sample;
-  const size_t smem = kVoteQueueBytes + vote_acc_words(a.chunk) * 4;
-  PPF_REQUIRE((int)smem <= ctx.vote_smem_limit, PPF_ERR_INTERNAL, "vote accumulator too large");
-  auto kernel = vote_kernel<false>;
-  PPF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  constexpr int kCands = sizeof(kSegShifts) / sizeof(kSegShifts[0]);
-  float best_ms[kCands];
-  for (int c = 0; c < kCands; ++c) best_ms[c] = INFINITY;
-  // two rounds over the candidates, the faster of each candidate's two times
-  for (int round = 0; round < 2; ++round)
-    for (int c = 0; c < kCands; ++c) {
-      a.seg_shift = kSegShifts[c];
-      PPF_CUDA(cudaMemsetAsync(cnt, 0, 64 + 32 + 80, stream));
-      PPF_CUDA(cudaEventRecord(ctx.ev[0], stream));
-      kernel<<<std::min<uint32_t>(sample, (uint32_t)sm_count()), kVoteThreads, smem, stream>>>(a);
-      PPF_CUDA(cudaGetLastError());
-      ctx.launches++;
-      PPF_CUDA(cudaEventRecord(ctx.ev[1], stream));
-      PPF_CUDA(cudaEventSynchronize(ctx.ev[1]));
-      float ms = 0;
-      PPF_CUDA(cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]));
-      best_ms[c] = std::min(best_ms[c], ms);
-    }
-  uint32_t flags = 0;
-  PPF_CUDA(cudaMemcpyAsync(&flags, cnt + 16, sizeof(flags), cudaMemcpyDeviceToHost, stream));
-  PPF_CUDA(cudaStreamSynchronize(stream));
-  PPF_REQUIRE(!(flags & kFlagBadIndex), PPF_ERR_INTERNAL, "vote kernel index out of range while tuning");
-  // the default stays unless another length is at least 2% faster
-  int pick = -1;
-  for (int c = 0; c < kCands; ++c)
-    if (kSegShifts[c] == kSegShiftDefault) pick = c;
-  for (int c = 0; c < kCands; ++c)
-    if (best_ms[c] < 0.98f * best_ms[pick]) pick = c;
-  m.seg_shift = kSegShifts[pick];
-  ctx.seg_tuned[signature] = m.seg_shift;
-}
-
 void pair_vote_counts(Context& ctx, const Model& m, const SceneData& s, uint64_t* out_dev) {
   VoteArgs a = make_args(m, s);
   dim3 grid((s.n + 255) / 256, std::min<uint32_t>(s.n, 65535u));
@@ -984,7 +1682,8 @@ void pair_vote_counts(Context& ctx, const Model& m, const SceneData& s, uint64_t
 // further cudaMalloc fails or takes memory the budget does not have) and
 // latency-bound loops that cannot take cudaMalloc/cudaFree latency or the
 // device-wide synchronisation that cudaFree implies.  Everything the pass
-// needs besides the caller's inputs and outputs lives in one static device
+// needs besides the caller's inputs and outputs lives in the context's 32-bit
+// counters, reserved when its models are built, and in one static device
 // array of this file, which every GPU that loads the library holds until the
 // process exits:
 //   [0, 256)        counters (the run_votes layout), the flags word at byte
@@ -1056,8 +1755,7 @@ void vote_cells_noalloc(Context& ctx, const Model& m, const float* xyz, const fl
               std::to_string(n_ref) + " scene reference points x " + std::to_string(m.t.n_chunks) +
                   " model chunks exceed the allocation-free limit of " + std::to_string(kNoAllocMaxItems) +
                   " work items");
-  const size_t smem = kVoteQueueBytes + vote_acc_words(m.t.chunk) * 4;
-  PPF_REQUIRE((int)smem <= ctx.vote_smem_limit, PPF_ERR_INTERNAL, "vote accumulator too large");
+  PPF_REQUIRE(ctx.vote_spill.ptr, PPF_ERR_INTERNAL, "vote counters not reserved");
 
   unsigned char* scratch = vote_scratch(ctx.device);
   cudaStream_t stream = ctx.stream;
@@ -1094,10 +1792,11 @@ void vote_cells_noalloc(Context& ctx, const Model& m, const float* xyz, const fl
   a.redo_items = reinterpret_cast<uint32_t*>(scratch + kNoAllocItemsOff);
   a.n_items_total = kNoAllocMaxItems;
   a.item_list = nullptr;
-  a.n_items = (uint32_t)n_items;
+  set_items(a, n_ref);
+  a.spill = ctx.vote_spill.as<uint2>();
+  a.n_items = (uint32_t)n_ref * a.n_cg;
   auto kernel = ctx.checks ? vote_kernel<true> : vote_kernel<false>;
-  PPF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<(unsigned)std::min<uint64_t>(n_items, (uint64_t)sm_count()), kVoteThreads, smem, stream>>>(a);
+  kernel<<<(unsigned)std::min<uint64_t>(a.n_items, (uint64_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
   PPF_CUDA(cudaGetLastError());
   ctx.launches++;
 
