@@ -19,7 +19,8 @@ namespace ppf {
 // outside that range must not matter to the caller's order.  A sort whose
 // look-back gave up leaves its output undefined (but every write inside the
 // buffers): sort() waits for the stream, reads the flag and raises
-// PPF_ERR_TIMEOUT, so nothing downstream reads that output.
+// PPF_ERR_TIMEOUT, so nothing downstream reads that output.  A sort of at most
+// 4096 elements runs in one block, without look-back and without waiting.
 template <typename K>
 class RadixSorter {
  public:
@@ -35,13 +36,13 @@ class RadixSorter {
     valt_.release();
     hist_.release();
     status_.release();
-    counters_.release();
   }
 
  private:
-  DevBuf kalt_, valt_, hist_, status_, counters_;
+  DevBuf kalt_, valt_, hist_, status_;
+  unsigned long long epoch_ = 0;  // passes since status_ was cleared
   size_t launches_ = 0;
-  bool stall_ = false;
+  bool stall_ = false, attributes_ = false;
 };
 
 extern template class RadixSorter<uint32_t>;
