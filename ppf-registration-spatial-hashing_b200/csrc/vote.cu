@@ -237,7 +237,8 @@ constexpr uint32_t kOffSlotKey = kOffEvK + kEvents;      // run | kExactGroup
 constexpr uint32_t kOffSlotCnt = kOffSlotKey + kSlots;   // events, then offset of the group
 constexpr uint32_t kOffPcRun = kOffSlotCnt + kSlots;     // piece: its run
 constexpr uint32_t kOffPcInf = kOffPcRun + kMaxPieces;   // piece: see piece_info
-constexpr uint32_t kOffAcc = (kOffPcInf + kMaxPieces + 31) / 32 * 32;  // counters, see kRowStride
+constexpr uint32_t kOffFlags = kOffPcInf + kMaxPieces;   // per warp: flagged events
+constexpr uint32_t kOffAcc = (kOffFlags + kVoteWarps * 8 + 31) / 32 * 32;  // counters, see kRowStride
 // over the pieces while the list is filled: per warp the scene pairs that
 // await their lookup
 constexpr uint32_t kNearLen = 64;
@@ -254,6 +255,8 @@ constexpr uint32_t kOffPcInc = kOffPcUnit + kMaxPieces + 1;
 constexpr uint32_t kTabWords = 60, kQueueLen = 32;
 constexpr uint32_t kOffTab = kOffSlotKey;
 constexpr uint32_t kOffQueue = kOffTab + kVoteWarps * kTabWords;
+// events of a swept piece with ambiguous votes in the current block, a bit each
+constexpr uint32_t kFlagWords = (kPieceEvents + 31) / 32;
 static_assert(kVoteWarps * (kTabWords + 2 * kQueueLen) <= 2 * kSlots, "tables and queues fit the slots");
 
 // Accumulator: plane j holds the 16-bit counters of bins (2j, 2j + 1) of every
@@ -329,6 +332,8 @@ extern __shared__ __align__(16) uint32_t smem[];
 
 // The warp's histogram table and queue.
 __device__ __forceinline__ uint32_t* warp_tab() { return smem + kOffTab + (threadIdx.x >> 5) * kTabWords; }
+static_assert(kFlagWords <= 8, "flag words per warp");
+__device__ __forceinline__ uint32_t* warp_flags() { return smem + kOffFlags + (threadIdx.x >> 5) * 8; }
 __device__ __forceinline__ uint32_t* warp_queue() { return smem + kOffQueue + (threadIdx.x >> 5) * 2 * kQueueLen; }
 
 __device__ __forceinline__ uint32_t wrap30(int b) { return (uint32_t)(b < 0 ? b + PPF_N_ANGLE : b); }
@@ -424,6 +429,42 @@ __device__ __forceinline__ uint32_t queue_votes(const VoteArgs& a, const VoteSha
   return qn;
 }
 
+// Queues the ambiguous votes of a block's flagged events (a bit each) and
+// clears the flags; returns the queue's length and the lane's ambiguous votes.
+// Out of line and called at a block's end, where its callers hold little in
+// registers: inside their loops it spilled a fifth of the sweep's accesses.
+template <bool kCheck>
+__device__ __noinline__ uint2 queue_flagged(const VoteArgs& a, const VoteShared& sh, uint32_t pos, uint32_t end,
+                                            uint32_t ev0, bool sweep, uint32_t qn) {
+  uint32_t* const flags = warp_flags();
+  uint32_t n_exact = 0;
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t wd = 0; wd < kFlagWords; ++wd) {
+    uint32_t left = flags[wd];
+    while (left) {
+      const uint32_t ev = ev0 + 32 * wd + __ffs(left) - 1;
+      left &= left - 1;
+      const uint32_t re = smem[kOffEvW + ev] & (kTurn - 1u);
+      uint32_t amb = 0;
+#pragma unroll
+      for (int k = 0; k < kPerLane; ++k) {
+        const uint32_t p = pos + 32u * k + (threadIdx.x & 31);
+        if (p < end && in_range<kCheck>(a, 28, p, a.P)) {
+          const uint32_t r = ((__ldg(a.entries + p) & (kTurn - 1u)) * PPF_N_ANGLE) & (kTurn - 1u);
+          if (((re - r + kMargin - 1u) & (kTurn - 1u)) < 2 * kMargin - 1) amb |= 1u << k;
+        }
+      }
+      n_exact += __popc(amb);
+      qn = queue_votes<kCheck>(a, sh, amb, pos, ev, sweep, qn);
+    }
+    __syncwarp();
+    flags[wd] = 0u;
+  }
+  __syncwarp();
+  return make_uint2(qn, n_exact);
+}
+
 // Entries [pos, pos + 128) of a unit that ends at `end`, kPerLane per lane
 // (the pad row past the end).
 __device__ __forceinline__ void load_block(const uint32_t* entries, uint32_t pos, uint32_t end,
@@ -449,9 +490,8 @@ __device__ __forceinline__ void load_block(const uint32_t* entries, uint32_t pos
 // lie among 30 consecutive ones: distinct banks or one broadcast) and adds 15
 // words of 16-bit pairs, one per plane.  Events that lie inside the block's
 // bucket range then move one vote for each entry beyond them.  Returns the
-// queue's length and the lane's ambiguous votes.  Out of line and without
-// calls of its own (as count_unit), so that neither the block's phases around
-// it nor a callee's saved registers spill in its loops.
+// queue's length and the lane's ambiguous votes.  Out of line (as count_unit),
+// so that the block's phases around it do not spill in its loops.
 template <bool kCheck>
 __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh, uint32_t start, uint32_t end,
                                            uint32_t ev0, uint32_t cnt, uint32_t qn) {
@@ -460,6 +500,7 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
   const uint32_t* const ev = smem + kOffEvW + ev0;
   uint32_t* const acc = smem + kOffAcc;
   uint32_t* const tab = warp_tab();
+  uint32_t* const flags = warp_flags();  // (all clear between units)
   const uint32_t rs = a.r_shift;
   const uint32_t* const entries = a.entries;  // (a copy: a's fields are read anew after every atomic)
   uint32_t passed = 0;  // events of a bucket below the block's first: counted in H as Q_s - 1
@@ -544,6 +585,7 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
     // events among the block's entries, and within the margin of one; a block
     // near R = 0 meets the margin across it and looks at every event
     const bool edge = rmin < kMargin || rmax > kTurn - kMargin;
+    bool flagged = false;
     for (uint32_t q = edge ? 0u : min(passed, done); q < cnt; ++q) {
       const uint32_t w = ev[q], re = w & (kTurn - 1u), qe = w >> PPF_ANGLE_BITS;
       if (!edge && (re >> rs) > b1 && re >= rmax + kMargin) break;
@@ -563,14 +605,15 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
         }
       }
       if (__any_sync(0xffffffffu, nearest < 2 * kMargin - 1)) {
-        uint32_t amb = 0;
-#pragma unroll
-        for (int k = 0; k < kPerLane; ++k)
-          if (rm[k] >= 0 && ((uint32_t)((int)re - rm[k] + (int)kMargin - 1) & (kTurn - 1u)) < 2 * kMargin - 1)
-            amb |= 1u << k;
-        n_exact += __popc(amb);
-        qn = queue_votes<kCheck>(a, sh, amb, pos, ev0 + q, true, qn);
+        flags[q >> 5] |= 1u << (q & 31);  // (all lanes write the same word)
+        flagged = true;
+        __syncwarp();
       }
+    }
+    if (flagged) {
+      const uint2 r = queue_flagged<kCheck>(a, sh, pos, end, ev0, true, qn);
+      qn = r.x;
+      n_exact += r.y;
     }
   }
   return make_uint2(qn, n_exact);
@@ -591,29 +634,34 @@ __device__ __noinline__ uint2 count_unit(const VoteArgs& a, const VoteShared& sh
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t* const entries = a.entries;
   uint32_t* const acc = smem + kOffAcc;
+  uint32_t* const flags = warp_flags();
   for (uint32_t pos = start; pos < end; pos += kBlock) {
     const uint32_t n = min((uint32_t)kBlock, end - pos);
     uint32_t c[kPerLane];
     load_block(entries, pos, end, c);
+    bool flagged = false;
     for (uint32_t g = 0; g < cnt; ++g) {
       const uint32_t base = count_angle(smem[kOffEvW + ev0 + g], 0u);
-      uint32_t amb = 0;
+      bool amb = false;  // (a lane past the end may say so too)
 #pragma unroll
       for (int k = 0; k < kPerLane; ++k) {
         if (32u * k < n && in_range<kCheck>(a, 14, c[k] >> PPF_ANGLE_BITS, kRowStride)) {
           const unsigned long long p = (unsigned long long)(base - (c[k] << kAngleShift)) * (PPF_N_ANGLE / 2);
           const uint32_t hi = (uint32_t)(p >> 32), lo = (uint32_t)p;
           atomicAdd(acc + hi * kRowStride + (c[k] >> PPF_ANGLE_BITS), 1u + (lo >> 31) * 65535u);
-          if ((lo << 1) > kSpan) amb |= 1u << k;
+          amb = amb || (lo << 1) > kSpan;
         }
       }
-      if (__any_sync(0xffffffffu, amb != 0u)) {
-#pragma unroll
-        for (int k = 0; k < kPerLane; ++k)
-          if (32u * k + lane >= n) amb &= ~(1u << k);
-        n_exact += __popc(amb);
-        qn = queue_votes<kCheck>(a, sh, amb, pos, ev0 + g, false, qn);
+      if (__any_sync(0xffffffffu, amb)) {
+        flags[g >> 5] |= 1u << (g & 31);
+        flagged = true;
+        __syncwarp();
       }
+    }
+    if (flagged) {
+      const uint2 r = queue_flagged<kCheck>(a, sh, pos, end, ev0, false, qn);
+      qn = r.x;
+      n_exact += r.y;
     }
   }
   return make_uint2(qn, n_exact);
@@ -943,6 +991,7 @@ __device__ __forceinline__ void vote_units(const VoteArgs& a, VoteShared& sh, Vo
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t* const pc_unit = smem + kOffPcUnit;
   if (tid == 0) sh.next = u0 + kVoteWarps;
+  if (lane < 8) warp_flags()[lane] = 0u;
   block_sync();
   uint32_t qn = 0;
   const uint32_t stride = (n_pieces + 31) / 32;
