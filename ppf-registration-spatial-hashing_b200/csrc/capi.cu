@@ -29,6 +29,8 @@ Context::~Context() {
   sort32.release();
   sort64.release();
   if (stream) cudaStreamSynchronize(stream);
+  if (host && host_pinned) cudaFreeHost(host);
+  else std::free(host);
   for (auto& e : ev)
     if (e) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
@@ -129,6 +131,7 @@ LookupOut finish_lookup(Context& ctx, Model& m, LookupState& st, const SceneData
     return out;
   }
   compute_poses(ctx, m, s, st);
+  uint32_t flags = 0;
   if (m.cpu_clustering) {
     float poses[48];
     uint32_t votes[3];
@@ -139,19 +142,16 @@ LookupOut finish_lookup(Context& ctx, Model& m, LookupState& st, const SceneData
     out.stats.max_idx = 0;
     out.stats.best_score = nc > 0 ? (float)votes[0] : 0.f;
     out.stats.cluster_path = 4;
+    PPF_CUDA(cudaEventRecord(ctx.ev[3], ctx.stream));
+    PPF_CUDA(cudaMemcpyAsync(ctx.host, ctx.flags.ptr, 4, cudaMemcpyDeviceToHost, ctx.stream));
+    PPF_CUDA(cudaStreamSynchronize(ctx.stream));
+    flags = ctx.host[0];
   } else {
     float best_score = 0;
-    size_t idx = cluster_poses_gpu(ctx, m, st, &best_score);
-    PPF_CUDA(cudaMemcpyAsync(out.pose, st.best.ptr, sizeof(out.pose), cudaMemcpyDeviceToHost, ctx.stream));
-    out.stats.max_idx = idx;
+    out.stats.max_idx = cluster_poses_gpu(ctx, m, st, out.pose, &best_score, &flags);
     out.stats.best_score = best_score;
     out.stats.cluster_path = st.cluster_path;
   }
-  PPF_CUDA(cudaEventRecord(ctx.ev[3], ctx.stream));
-  PPF_CUDA(cudaStreamSynchronize(ctx.stream));
-  uint32_t flags = 0;
-  PPF_CUDA(cudaMemcpyAsync(&flags, ctx.flags.ptr, 4, cudaMemcpyDeviceToHost, ctx.stream));
-  PPF_CUDA(cudaStreamSynchronize(ctx.stream));
   PPF_REQUIRE(!(flags & kFlagSpinTimeout), PPF_ERR_TIMEOUT, "radix sort look-back timed out");
   PPF_CUDA(cudaEventElapsedTime(&out.stats.total_ms, ctx.ev[2], ctx.ev[3]));
   out.stats.gpu_launches = (uint32_t)(ctx.launches - launches0);
@@ -216,7 +216,7 @@ void check_cloud(const float* xyz, const float* nxyz, uint64_t n) {
   PPF_REQUIRE(n >= 1, PPF_ERR_INVALID_ARGUMENT, "empty cloud");
 }
 
-void init_context(Context& c, int device) {
+void init_context(Context& c, int device, bool kept) {
   int count = 0;
   PPF_CUDA(cudaGetDeviceCount(&count));
   PPF_REQUIRE(count > 0, PPF_ERR_CUDA, "no CUDA device");
@@ -229,6 +229,13 @@ void init_context(Context& c, int device) {
   PPF_CUDA(cudaDeviceGetDefaultMemPool(&pool, c.device));
   uint64_t keep = UINT64_MAX;
   PPF_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  if (kept) {
+    PPF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c.host), kHostBytes, cudaHostAllocPortable));
+    c.host_pinned = true;
+  } else {
+    c.host = static_cast<uint32_t*>(std::malloc(kHostBytes));
+    if (!c.host) throw std::bad_alloc();
+  }
   StreamScope scope(c.stream);
   c.flags.reserve(256);
   c.counters.reserve(256);
@@ -600,7 +607,7 @@ ppf_status ppf_registration(ppf_context_t ctx, uint64_t n_scenes, const float* c
     ppf_context_t c = ctx;
     if (!c) {
       std::unique_ptr<ppf_context_s> fresh(new ppf_context_s());
-      init_context(fresh->c, dev_use);
+      init_context(fresh->c, dev_use, false);
       own.reset(fresh.release());
       c = own.get();
     }

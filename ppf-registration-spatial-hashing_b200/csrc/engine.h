@@ -36,6 +36,8 @@ constexpr uint32_t kFlagRows = 1024;
 
 // Every DevBuf member must be released in ~Context (capi.cu) before the
 // stream its blocks are freed on is destroyed.
+constexpr size_t kHostBytes = 4096;
+
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -43,6 +45,12 @@ struct Context {
   RadixSorter<unsigned long long> sort64;
   DevBuf flags;      // uint32 device flags (kFlag*)
   DevBuf counters;   // small device counters for kernels
+  // Host memory that small results are copied to (kHostBytes).  Pinned in a
+  // context that is kept: a copy to pageable memory is staged and waits on its
+  // own (about 5 us each).  Pinning takes 0.5 ms, so a context made for one
+  // call does without.
+  uint32_t* host = nullptr;
+  bool host_pinned = false;
   DevBuf scratch;    // run-table scratch
   // vote-pass candidate cells (code, count), kept and grown across lookups
   DevBuf cand_codes, cand_counts, redo_items;
@@ -96,6 +104,10 @@ struct ModelTables {
   // run.  lut_quantum: the quantum they hold for (0: no table)
   DevBuf lut, row_flags;
   float lut_quantum = 0;
+  // |t - s|^2 < x_star equals sqrtf(|t - s|^2) < d_dist on the device
+  // (dist_threshold_kernel), if x_star_ok
+  float x_star = 0;
+  bool x_star_ok = false;
   // m_r chunking of the vote accumulator
   uint32_t chunk = 0, n_chunks = 0;
   DevBuf split;  // uint32 [K * (n_chunks + 1)] first run position per chunk
@@ -213,8 +225,14 @@ size_t select_votes(Context& ctx, const Model& m, const SceneData& s, LookupStat
 // Orders arbitrary (code, count) pairs by code ascending (all-votes dump).
 void sort_by_code(Context& ctx, LookupState& st, size_t n);
 void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState& st);
-// GPU clustering + argmax; writes the best pose into st.best and returns the index.
-size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* best_score);
+// GPU clustering + argmax; writes the best pose (16 floats) and its score and
+// returns the index.  Records ctx.ev[3] and waits for the stream; *flags
+// receives the device flags as of then.
+size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* pose, float* best_score,
+                         uint32_t* flags);
+// Threshold of the clustering's translation test for cells of size d: out[0]
+// its float bits, out[1] nonzero if it cannot be used (both zero before).
+void calibrate_distance(Context& ctx, float d, uint32_t* out_dev);
 
 // ---- driver preprocessing (preprocess.cu)
 // per-axis min / max over finite points (false when there is none)
@@ -234,7 +252,7 @@ struct LookupOut {
   ppf_stats stats{};
   size_t cand_hint = 0;  // candidate cells to provide for the next pass of this model
 };
-void init_context(Context& c, int device);
+void init_context(Context& c, int device, bool kept = true);
 // Lookups of (models[i], scenes[i]) with one batched vote pass.  states:
 // per-request lookup state (nullptr: each model's own `last`); caps:
 // per-request candidate capacity hints (nullptr: the models' last passes).

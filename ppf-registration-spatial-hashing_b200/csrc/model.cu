@@ -2,6 +2,7 @@
 // pair features and keys of all ordered model pairs, a stable key sort, run
 // tables, per-pair vote entries and the key -> run lookup table.
 #include <algorithm>
+#include <cstring>
 
 #include "engine.h"
 #include "ppf_math.cuh"
@@ -512,11 +513,16 @@ void build_model(Context& ctx, ModelTables& t, const float* xyz, const float* nx
         t.n_chunks, t.split.as<uint32_t>(), bad, ctx.flags.as<uint32_t>());
     PPF_CUDA(cudaGetLastError());
   }
-  uint32_t flags = 0;
+  PPF_CUDA(cudaMemsetAsync(ctx.counters.ptr, 0, 8, st));
+  calibrate_distance(ctx, d_dist, ctx.counters.as<uint32_t>());
   unsigned long long badh[2] = {0, 0};
-  PPF_CUDA(cudaMemcpyAsync(&flags, ctx.flags.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  PPF_CUDA(cudaMemcpyAsync(ctx.host, ctx.flags.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  PPF_CUDA(cudaMemcpyAsync(ctx.host + 2, ctx.counters.ptr, 8, cudaMemcpyDeviceToHost, st));
   if (ctx.checks) PPF_CUDA(cudaMemcpyAsync(badh, bad, 16, cudaMemcpyDeviceToHost, st));
   PPF_CUDA(cudaStreamSynchronize(st));
+  const uint32_t flags = ctx.host[0];
+  std::memcpy(&t.x_star, ctx.host + 2, sizeof(t.x_star));
+  t.x_star_ok = ctx.host[3] == 0;
   PPF_REQUIRE(!(flags & kFlagSpinTimeout), PPF_ERR_TIMEOUT, "radix sort look-back timed out");
   PPF_REQUIRE(!(flags & kFlagBadIndex), PPF_ERR_INTERNAL,
               "model tables inconsistent: check " + std::to_string(badh[0]) + " at " +

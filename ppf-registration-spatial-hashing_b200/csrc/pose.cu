@@ -94,6 +94,40 @@ __global__ void gather_packed_kernel(const uint32_t* __restrict__ perm, const K*
   }
 }
 
+// Keep and order in one key: the kept votes' max_count - count above their
+// packed codes (code_bits bits), so that one sort gives count descending, then
+// code ascending.
+__global__ void filter_keys_kernel(const unsigned long long* __restrict__ code, const uint32_t* __restrict__ count,
+                                   size_t n, float min_votecount, uint32_t max_count, int kb, int code_bits,
+                                   unsigned long long* __restrict__ out, uint32_t* __restrict__ n_out) {
+  const int lane = threadIdx.x & 31;
+  for (size_t b = blockIdx.x * (size_t)blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = b + threadIdx.x;
+    const uint32_t cnt = i < n ? count[i] : 0u;
+    const bool keep = i < n && (float)cnt > min_votecount;
+    const uint32_t ballot = __ballot_sync(0xffffffffu, keep);
+    if (!ballot) continue;
+    uint32_t s0 = 0;
+    if (lane == 0) s0 = atomicAdd(n_out, (uint32_t)__popc(ballot));
+    s0 = __shfl_sync(0xffffffffu, s0, 0);
+    if (keep) {
+      const unsigned long long c = code[i];
+      out[s0 + __popc(ballot & ((1u << lane) - 1u))] =
+          (unsigned long long)(max_count - cnt) << code_bits | ((c >> 32) << kb) | (uint32_t)c;
+    }
+  }
+}
+
+__global__ void split_keys_kernel(const unsigned long long* __restrict__ key, size_t n, uint32_t max_count, int kb,
+                                  int code_bits, unsigned long long* __restrict__ code,
+                                  uint32_t* __restrict__ count) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const unsigned long long k = key[i], c = k & ((1ull << code_bits) - 1);
+    code[i] = ((c >> kb) << 32) | (c & ((1ull << kb) - 1));
+    count[i] = max_count - (uint32_t)(k >> code_bits);
+  }
+}
+
 struct PoseArgs {
   const unsigned long long* codes;
   const uint32_t* counts;
@@ -109,6 +143,7 @@ struct PoseArgs {
   float* quats;
   float* weighted;
   uint32_t* cell_keys;
+  uint32_t* cells_sorted;  // cell_keys again, to be sorted
   uint32_t* adj;
   int4* cells3;
 };
@@ -148,7 +183,9 @@ __global__ void poses_kernel(PoseArgs a) {
     a.quats[4 * i + 3] = q.w;
     a.weighted[i] = a.m_w[mr] * a.counts[i];
     int3 c = trans_cell(t, a.d_dist);
-    a.cell_keys[i] = cell_key(c.x, c.y, c.z);
+    const uint32_t key = cell_key(c.x, c.y, c.z);
+    a.cell_keys[i] = key;
+    a.cells_sorted[i] = key;
     a.cells3[i] = make_int4(c.x, c.y, c.z, 0);
     uint32_t* adj = a.adj + 27 * i;
     int idx = 0;
@@ -227,25 +264,58 @@ __global__ void cluster_kernel(ClusterArgs a) {
 
 constexpr int kGroup = 32;  // clustering targets per warp
 
-// Also folds the largest squared norm of a finite quaternion into *max_qq
-// (float bits; non-negative floats order as their bits).
-__global__ void gather_sorted_kernel(const uint32_t* __restrict__ map, size_t U,
-                                     const float* __restrict__ quats, const float* __restrict__ trans0,
-                                     const float* __restrict__ weighted, float4* __restrict__ qs,
-                                     float4* __restrict__ tws, uint32_t* __restrict__ max_qq) {
+// What the clustering needs to know of all poses before it is chosen.
+struct ClusterChecks {
+  // two different int3 cells share one cell key (then the per-pose neighbour
+  // lists of cluster_kernel are needed): a sorted position whose key equals
+  // its predecessor's but whose cell differs
+  uint32_t mixed;
+  uint32_t groups, items32;       // work items of the warp and split clustering
+  uint32_t nonint;                // some weight is not an integer below 2^24 (or is NaN)
+  unsigned long long abs_sum;     // sum of |weight| over all poses
+  uint32_t max_qq;                // largest squared norm of a finite quaternion (float bits)
+  uint32_t runs;                  // cells
+};
+
+// Poses in cell order, and the checks over them.
+__global__ void gather_sorted_kernel(const uint32_t* __restrict__ sorted_keys, const uint32_t* __restrict__ map,
+                                     const int4* __restrict__ cells3, size_t U, const float* __restrict__ quats,
+                                     const float* __restrict__ trans0, const float* __restrict__ weighted,
+                                     float4* __restrict__ qs, float4* __restrict__ tws, bool weights,
+                                     ClusterChecks* __restrict__ checks) {
   float m = 0.f;
+  bool mixed = false, nonint = false;
+  unsigned long long sum = 0;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < U;
        p += (size_t)gridDim.x * blockDim.x) {
     uint32_t o = map[p];
     const float4 q = make_float4(quats[4 * o], quats[4 * o + 1], quats[4 * o + 2], quats[4 * o + 3]);
+    const float w = weighted[o], aw = fabsf(w);
     qs[p] = q;
-    tws[p] = make_float4(trans0[3 * o], trans0[3 * o + 1], trans0[3 * o + 2], weighted[o]);
+    tws[p] = make_float4(trans0[3 * o], trans0[3 * o + 1], trans0[3 * o + 2], w);
+    // non-negative floats order as their bits
     const float qq = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
     if (isfinite(qq)) m = fmaxf(m, qq);
+    if (!(aw < 16777216.f) || w != truncf(w)) nonint = true;
+    else sum += (unsigned long long)aw;
+    if (p && sorted_keys[p] == sorted_keys[p - 1]) {
+      const int4 c = cells3[o], c0 = cells3[map[p - 1]];
+      mixed = mixed || c.x != c0.x || c.y != c0.y || c.z != c0.z;
+    }
   }
+  mixed = __any_sync(0xffffffffu, mixed);
+  nonint = __any_sync(0xffffffffu, nonint);
 #pragma unroll
-  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(max_qq, __float_as_uint(m));
+  for (int o = 16; o; o >>= 1) {
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (weights) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (m > 0.f) atomicMax(&checks->max_qq, __float_as_uint(m));
+    if (mixed) atomicOr(&checks->mixed, 1u);
+    if (nonint) atomicOr(&checks->nonint, 1u);
+    if (weights && sum) atomicAdd(&checks->abs_sum, sum);
+  }
 }
 
 // Quaternion half-width of the box filters.  The reference's rotation test
@@ -257,19 +327,6 @@ float quat_margin(float max_qq) {
   const double rot_sq = (double)(2 * PPF_D_ANGLE_HOST) * (double)(2 * PPF_D_ANGLE_HOST);
   const double r2 = std::max(0.0, 2.0 * (double)max_qq - 2.0);
   return (float)(std::sqrt(r2 + rot_sq / 4.0 + 1e-5) + 1e-5);
-}
-
-// Whether two different int3 cells share one cell key (then the per-pose
-// neighbour lists of cluster_kernel are needed): a sorted position whose key
-// equals its predecessor's but whose cell differs.
-__global__ void mixed_cells_kernel(const uint32_t* __restrict__ sorted_keys, const uint32_t* __restrict__ map,
-                                   const int4* __restrict__ cells3, size_t U, uint32_t* __restrict__ mixed) {
-  for (size_t p = 1 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < U;
-       p += (size_t)gridDim.x * blockDim.x) {
-    if (sorted_keys[p] != sorted_keys[p - 1]) continue;
-    const int4 c = cells3[map[p]], c0 = cells3[map[p - 1]];
-    if (c.x != c0.x || c.y != c0.y || c.z != c0.z) atomicOr(mixed, 1u);
-  }
 }
 
 // 4-D grid bucket of a unit quaternion, 16 cells of 0.125 per component.
@@ -287,7 +344,8 @@ __device__ __forceinline__ uint32_t quat_bucket(float4 q) {
 constexpr int kTargetKeyBits = 54;
 __global__ void target_keys_kernel(const uint32_t* __restrict__ sorted_keys, const float4* __restrict__ qs,
                                    const float4* __restrict__ tws, float sub_scale, size_t U,
-                                   unsigned long long* __restrict__ keys) {
+                                   unsigned long long* __restrict__ keys, const float* __restrict__ trans0,
+                                   float* __restrict__ scores, float* __restrict__ trans) {
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < U;
        p += (size_t)gridDim.x * blockDim.x) {
     const float4 tw = tws[p];
@@ -295,6 +353,12 @@ __global__ void target_keys_kernel(const uint32_t* __restrict__ sorted_keys, con
                          ((uint32_t)__float2int_rd(tw.y * sub_scale) & 3u) << 2 |
                          ((uint32_t)__float2int_rd(tw.z * sub_scale) & 3u);
     keys[p] = ((unsigned long long)sorted_keys[p] << 22) | ((unsigned long long)quat_bucket(qs[p]) << 6) | sub;
+    if (scores) {  // split clustering: scores start at 1 (the pose itself), translations stay the snapshot's
+      scores[p] = 1.f;
+      trans[3 * p] = trans0[3 * p];
+      trans[3 * p + 1] = trans0[3 * p + 1];
+      trans[3 * p + 2] = trans0[3 * p + 2];
+    }
   }
 }
 
@@ -339,10 +403,12 @@ __global__ void dist_threshold_kernel(float d, uint32_t* __restrict__ out) {
 // 32-target groups and, if items32 is set, the number of split items (32-target
 // tiles x 27 neighbours).
 __global__ void run_adjacency_kernel(const uint32_t* __restrict__ first, const uint32_t* __restrict__ count,
-                                     size_t Kc, const uint32_t* __restrict__ map,
+                                     size_t Kc, const uint32_t* __restrict__ kc_dev,
+                                     const uint32_t* __restrict__ map,
                                      const int4* __restrict__ cells3, const uint32_t* __restrict__ uniq,
                                      int* __restrict__ adjrun, uint32_t* __restrict__ groups,
                                      uint32_t* __restrict__ items32) {
+  if (kc_dev) Kc = *kc_dev;  // (Kc is then an upper bound)
   for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < Kc;
        r += (size_t)gridDim.x * blockDim.x) {
     const uint32_t f = first[r], n = count[r];
@@ -609,37 +675,6 @@ __global__ void __launch_bounds__(kWarpBlock, 8) cluster_warp_kernel(GroupArgs a
 // as cluster_warp_kernel, and adds its partial sum with a float atomic.  A
 // lookup with few poses then spreads over up to 27x more warps.
 
-// nonint: some weight is not an integer below 2^24 (or is NaN); abs_sum: the
-// sum of |weight| over all poses.
-__global__ void weight_check_kernel(const float* __restrict__ w, size_t U, uint32_t* __restrict__ nonint,
-                                    unsigned long long* __restrict__ abs_sum) {
-  unsigned long long s = 0;
-  bool bad = false;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < U; i += (size_t)gridDim.x * blockDim.x) {
-    const float x = w[i], ax = fabsf(x);
-    if (!(ax < 16777216.f) || x != truncf(x)) bad = true;
-    else s += (unsigned long long)ax;
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  bad = __any_sync(0xffffffffu, bad);
-  if ((threadIdx.x & 31) == 0) {
-    if (bad) atomicOr(nonint, 1u);
-    if (s) atomicAdd(abs_sum, s);
-  }
-}
-
-// Scores start at 1 (the pose itself); translations stay the snapshot's.
-__global__ void split_init_kernel(size_t U, const float* __restrict__ trans0, float* __restrict__ scores,
-                                  float* __restrict__ trans) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < U; i += (size_t)gridDim.x * blockDim.x) {
-    scores[i] = 1.f;
-    trans[3 * i] = trans0[3 * i];
-    trans[3 * i + 1] = trans0[3 * i + 1];
-    trans[3 * i + 2] = trans0[3 * i + 2];
-  }
-}
-
 constexpr int kSplitBlock = 256;
 
 __global__ void __launch_bounds__(kSplitBlock) cluster_split_kernel(GroupArgs a) {
@@ -783,19 +818,6 @@ size_t select_votes(Context& ctx, const Model& m, const SceneData& s, LookupStat
                     const unsigned long long* cand_code, const uint32_t* cand_count, size_t n_cand,
                     float min_votecount, uint32_t max_count) {
   cudaStream_t stream = ctx.stream;
-  unsigned long long* fcode = grow<unsigned long long>(st.tmp64, n_cand + 1);
-  uint32_t* fcount = grow<uint32_t>(st.tmp32a, n_cand + 1);
-  PPF_CUDA(cudaMemsetAsync(ctx.counters.ptr, 0, 4, stream));
-  filter_kernel<<<grid_for(n_cand, 256), 256, 0, stream>>>(
-      cand_code, cand_count, n_cand, min_votecount,
-      fcode, fcount, ctx.counters.as<uint32_t>());
-  PPF_CUDA(cudaGetLastError());
-  ctx.launches++;
-  uint32_t U = 0;
-  PPF_CUDA(cudaMemcpyAsync(&U, ctx.counters.ptr, 4, cudaMemcpyDeviceToHost, stream));
-  PPF_CUDA(cudaStreamSynchronize(stream));
-  st.U = U;
-  if (U == 0) return 0;
   // code ascending (codes are unique), counts carried as values; codes are
   // packed to the bits that s_r and m_r need
   auto bits_for = [](uint64_t x) {
@@ -805,7 +827,40 @@ size_t select_votes(Context& ctx, const Model& m, const SceneData& s, LookupStat
   };
   const int kb = 6 + bits_for(m.t.n > 1 ? m.t.n - 1 : 1);
   const int code_bits = kb + bits_for(s.n > 1 ? s.n - 1 : 1);
-  PPF_CUDA(cudaMemsetAsync(ctx.flags.ptr, 0, 4, stream));
+  const int key_bits = code_bits + std::max(1, bits_for(max_count));
+  unsigned long long* fcode = grow<unsigned long long>(st.tmp64, n_cand + 1);
+  uint32_t* fcount = grow<uint32_t>(st.tmp32a, n_cand + 1);
+  // counter 0: kept votes; from counter 2: ClusterChecks of cluster_poses_gpu
+  PPF_CUDA(cudaMemsetAsync(ctx.counters.ptr, 0, 64, stream));
+  auto read_count = [&]() {
+    PPF_CUDA(cudaMemcpyAsync(ctx.host, ctx.counters.ptr, 4, cudaMemcpyDeviceToHost, stream));
+    PPF_CUDA(cudaStreamSynchronize(stream));
+    return (size_t)ctx.host[0];
+  };
+  if (max_count < (1u << 24) && key_bits <= 64) {
+    filter_keys_kernel<<<grid_for(n_cand, 256), 256, 0, stream>>>(cand_code, cand_count, n_cand, min_votecount,
+                                                                  max_count, kb, code_bits, fcode,
+                                                                  ctx.counters.as<uint32_t>());
+    PPF_CUDA(cudaGetLastError());
+    ctx.launches++;
+    const size_t U = st.U = read_count();
+    if (U == 0) return 0;
+    const size_t l0 = ctx.sort64.launches();
+    ctx.sort64.sort(fcode, fcount, true, U, 0, key_bits, stream, ctx.flags.as<uint32_t>());
+    split_keys_kernel<<<grid_for(U, 256), 256, 0, stream>>>(fcode, U, max_count, kb, code_bits,
+                                                            grow<unsigned long long>(st.codes, U),
+                                                            grow<uint32_t>(st.counts, U));
+    PPF_CUDA(cudaGetLastError());
+    ctx.launches += 1 + (ctx.sort64.launches() - l0);
+    return U;
+  }
+  filter_kernel<<<grid_for(n_cand, 256), 256, 0, stream>>>(
+      cand_code, cand_count, n_cand, min_votecount,
+      fcode, fcount, ctx.counters.as<uint32_t>());
+  PPF_CUDA(cudaGetLastError());
+  ctx.launches++;
+  const size_t U = st.U = read_count();
+  if (U == 0) return 0;
   size_t l0 = ctx.sort64.launches() + ctx.sort32.launches();
   uint32_t* packed32 = nullptr;
   if (code_bits <= 32) {
@@ -870,6 +925,7 @@ void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState
   a.quats = grow<float>(st.quats, U * 4);
   a.weighted = grow<float>(st.weighted, U);
   a.cell_keys = grow<uint32_t>(st.cell_keys, U);
+  a.cells_sorted = grow<uint32_t>(st.cells_sorted, U);
   a.adj = grow<uint32_t>(st.adj, U * 27);
   a.cells3 = grow<int4>(st.cells3, U);
   grow<float>(st.trans, U * 3);
@@ -892,28 +948,56 @@ void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState
   ctx.launches++;
 }
 
-size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* best_score) {
+void calibrate_distance(Context& ctx, float d, uint32_t* out_dev) {
+  dist_threshold_kernel<<<(2 * kDistWindow + 1 + 255) / 256, 256, 0, ctx.stream>>>(d, out_dev);
+  PPF_CUDA(cudaGetLastError());
+  ctx.launches++;
+}
+
+size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* pose, float* best_score,
+                         uint32_t* flags) {
   const size_t U = st.U;
   cudaStream_t stream = ctx.stream;
   float* best = grow<float>(st.best, 32);
   st.cluster_path = 0;
+  // best pose, score and index and the device flags, one wait for all
+  auto finish = [&]() {
+    PPF_CUDA(cudaEventRecord(ctx.ev[3], stream));
+    PPF_CUDA(cudaMemcpyAsync(ctx.host, best, 20 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    PPF_CUDA(cudaMemcpyAsync(ctx.host + 20, ctx.flags.ptr, 4, cudaMemcpyDeviceToHost, stream));
+    PPF_CUDA(cudaStreamSynchronize(stream));
+    std::memcpy(pose, ctx.host, 16 * sizeof(float));
+    std::memcpy(best_score, ctx.host + 16, sizeof(float));
+    *flags = ctx.host[20];
+    unsigned long long idx;
+    std::memcpy(&idx, ctx.host + 18, sizeof(idx));
+    return (size_t)idx;
+  };
   if (U <= 1) {
     PPF_CUDA(cudaMemsetAsync(best, 0, 32 * sizeof(float), stream));
-    *best_score = 0;
-    return 0;
+    return finish();
   }
+  ClusterChecks* const checks = reinterpret_cast<ClusterChecks*>(ctx.counters.as<uint32_t>() + 2);
+  static_assert(8 + sizeof(ClusterChecks) <= 64, "the checks fit the counters that select_votes cleared");
   // hash array of the pose cells (src/cuda/model.cu:222-226)
-  uint32_t* ck = grow<uint32_t>(st.cells_sorted, U);
+  uint32_t* ck = st.cells_sorted.as<uint32_t>();  // cell keys, by compute_poses
   uint32_t* map = grow<uint32_t>(st.cells_map, U);
-  PPF_CUDA(cudaMemcpyAsync(ck, st.cell_keys.ptr, U * 4, cudaMemcpyDeviceToDevice, stream));
-  PPF_CUDA(cudaMemsetAsync(ctx.flags.ptr, 0, 4, stream));
   size_t l0 = ctx.sort32.launches();
   ctx.sort32.sort(ck, map, true, U, 0, 32, stream, ctx.flags.as<uint32_t>());
   ctx.launches += ctx.sort32.launches() - l0;
   uint32_t* uq = grow<uint32_t>(st.cells_uniq, U);
   uint32_t* fi = grow<uint32_t>(st.cells_first, U);
   uint32_t* ct = grow<uint32_t>(st.cells_count, U);
-  size_t Kc = build_runs(ck, U, uq, fi, ct, ctx.scratch, stream, &ctx.launches);
+  // Few poses: one launch, and the number of cells stays on the device until
+  // the checks are read (tables sized for a cell per pose).
+  const bool few = U <= kRunsSmall;
+  size_t Kc = U;
+  if (few) {
+    build_runs_small(ck, U, uq, fi, ct, &checks->runs, stream);
+    ctx.launches++;
+  } else {
+    Kc = build_runs(ck, U, uq, fi, ct, ctx.scratch, stream, &ctx.launches);
+  }
   ClusterArgs a;
   a.U = U;
   a.trans0 = st.trans0.as<float>();
@@ -924,7 +1008,6 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
   a.first = fi;
   a.count = ct;
   a.map = map;
-  a.Kc = Kc;
   a.d_dist = m.t.d_dist;
   a.use_l1 = m.use_l1_norm;
   a.use_avg = m.use_averaged_clusters;
@@ -940,52 +1023,39 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
   // they are exact in any order (integer weights, absolute sum below 2^24).
   const bool may_split = ctx.cluster_split && !m.use_averaged_clusters;
   uint32_t* item_off32 = may_split ? grow<uint32_t>(st.item_off32, Kc + 1) : nullptr;
-  // counters: [0] mixed cells, [1] tiles, [2] split items, [3] non-integer
-  // weight, [4..5] sum of |weight|, [6] largest squared quaternion norm,
-  // [7] x_star of the translation test, [8] x_star unusable
-  PPF_CUDA(cudaMemsetAsync(ctx.counters.ptr, 0, 36, stream));
-  uint32_t* mixed = ctx.counters.as<uint32_t>();
   const float d_dist = m.t.d_dist;
-  const bool calibrate = !m.use_l1_norm && d_dist > 0.f && std::isfinite(d_dist);
-  if (calibrate) {
-    dist_threshold_kernel<<<(2 * kDistWindow + 1 + 255) / 256, 256, 0, stream>>>(d_dist, mixed + 7);
-    ctx.launches++;
-  }
-  gather_sorted_kernel<<<grid_for(U, 256), 256, 0, stream>>>(map, U, a.quats, a.trans0, a.weighted, qs, tws,
-                                                              mixed + 6);
-  mixed_cells_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, map, st.cells3.as<int4>(), U, mixed);
-  run_adjacency_kernel<<<grid_for(Kc, 128), 128, 0, stream>>>(fi, ct, Kc, map, st.cells3.as<int4>(), uq,
+  gather_sorted_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, map, st.cells3.as<int4>(), U, a.quats, a.trans0,
+                                                              a.weighted, qs, tws, may_split, checks);
+  const uint32_t* kc_dev = few ? &checks->runs : nullptr;
+  run_adjacency_kernel<<<grid_for(Kc, 128), 128, 0, stream>>>(fi, ct, Kc, kc_dev, map, st.cells3.as<int4>(), uq,
                                                               adjrun, item_off, item_off32);
-  exclusive_scan_small(item_off, Kc, mixed + 1, stream);
-  ctx.launches += 4;
-  if (may_split) {
-    exclusive_scan_small(item_off32, Kc, mixed + 2, stream);
-    weight_check_kernel<<<grid_for(U, 256), 256, 0, stream>>>(a.weighted, U, mixed + 3,
-                                                              reinterpret_cast<unsigned long long*>(mixed + 4));
-    ctx.launches += 2;
-  }
-  uint32_t hc[9];
-  PPF_CUDA(cudaMemcpyAsync(hc, mixed, sizeof(hc), cudaMemcpyDeviceToHost, stream));
+  exclusive_scan_small(item_off, item_off32, Kc, kc_dev, &checks->groups, stream);
+  PPF_CUDA(cudaGetLastError());
+  ctx.launches += 3;
+  PPF_CUDA(cudaMemcpyAsync(ctx.host, checks, sizeof(ClusterChecks), cudaMemcpyDeviceToHost, stream));
   PPF_CUDA(cudaStreamSynchronize(stream));
-  float max_qq, x_star;
-  std::memcpy(&max_qq, hc + 6, sizeof(max_qq));
-  std::memcpy(&x_star, hc + 7, sizeof(x_star));
+  ClusterChecks hc;
+  std::memcpy(&hc, ctx.host, sizeof(hc));
+  if (few) Kc = hc.runs;
+  a.Kc = Kc;
+  float max_qq;
+  std::memcpy(&max_qq, &hc.max_qq, sizeof(max_qq));
   const float qmargin = quat_margin(max_qq);
-  const int use_x_star = calibrate && !hc[8] && !ctx.cluster_sqrt;
+  const float x_star = m.t.x_star;
+  const int use_x_star = !m.use_l1_norm && m.t.x_star_ok && !ctx.cluster_sqrt;
   // quarter-cell translation bins of the target order
   const float sub_scale = d_dist > 0.f && std::isfinite(d_dist) ? 4.f / d_dist : 0.f;
-  const unsigned long long abs_sum = hc[4] | ((unsigned long long)hc[5] << 32);
-  const bool split = may_split && !hc[0] && !hc[3] && abs_sum < (1ull << 24) - 1;
-  st.cluster_path = split ? 3 : hc[0] ? 2 : 1;
+  const bool split = may_split && !hc.mixed && !hc.nonint && hc.abs_sum < (1ull << 24) - 1;
+  st.cluster_path = split ? 3 : hc.mixed ? 2 : 1;
   if (split) {
     // targets of each cell ordered by rotation bucket, as below
     unsigned long long* tkeys = grow<unsigned long long>(st.tmp64, U);
     uint32_t* tperm = grow<uint32_t>(st.tperm, U);
-    target_keys_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, qs, tws, sub_scale, U, tkeys);
+    target_keys_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, qs, tws, sub_scale, U, tkeys, a.trans0, a.scores,
+                                                             a.trans);
     const size_t l1 = ctx.sort64.launches();
     ctx.sort64.sort(tkeys, tperm, true, U, 0, kTargetKeyBits, stream, ctx.flags.as<uint32_t>());
     ctx.launches += 1 + ctx.sort64.launches() - l1;
-    split_init_kernel<<<grid_for(U, 256), 256, 0, stream>>>(U, a.trans0, a.scores, a.trans);
     GroupArgs ta;
     ta.tperm = tperm;
     ta.first = fi;
@@ -994,7 +1064,7 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
     ta.adjrun = adjrun;
     ta.item_off = item_off32;
     ta.Kc = Kc;
-    ta.n_items = hc[2];
+    ta.n_items = hc.items32;
     ta.qs = qs;
     ta.tws = tws;
     ta.d_dist = m.t.d_dist;
@@ -1005,17 +1075,18 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
     ta.use_avg = 0;
     ta.scores = a.scores;
     ta.trans = a.trans;
-    const size_t blocks = (hc[2] + kSplitBlock / 32 - 1) / (kSplitBlock / 32);
+    const size_t blocks = (hc.items32 + kSplitBlock / 32 - 1) / (kSplitBlock / 32);
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>(blocks, (size_t)sm_count() * 8));
     cluster_split_kernel<<<grid, kSplitBlock, 0, stream>>>(ta);
-    ctx.launches += 2;
-  } else if (hc[0]) {
+    ctx.launches++;
+  } else if (hc.mixed) {
     cluster_kernel<<<grid_for(U, 128), 128, 0, stream>>>(a);
   } else {
     // targets of each cell ordered by rotation bucket
     unsigned long long* tkeys = grow<unsigned long long>(st.tmp64, U);
     uint32_t* tperm = grow<uint32_t>(st.tperm, U);
-    target_keys_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, qs, tws, sub_scale, U, tkeys);
+    target_keys_kernel<<<grid_for(U, 256), 256, 0, stream>>>(ck, qs, tws, sub_scale, U, tkeys, nullptr, nullptr,
+                                                             nullptr);
     ctx.launches++;
     const size_t l1 = ctx.sort64.launches();
     ctx.sort64.sort(tkeys, tperm, true, U, 0, kTargetKeyBits, stream, ctx.flags.as<uint32_t>());
@@ -1028,7 +1099,7 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
     ta.adjrun = adjrun;
     ta.item_off = item_off;
     ta.Kc = Kc;
-    ta.n_items = hc[1];
+    ta.n_items = hc.groups;
     ta.qs = qs;
     ta.tws = tws;
     ta.d_dist = m.t.d_dist;
@@ -1039,7 +1110,7 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
     ta.use_avg = m.use_averaged_clusters;
     ta.scores = a.scores;
     ta.trans = a.trans;
-    const size_t blocks = (hc[1] + kWarpBlock / 32 - 1) / (kWarpBlock / 32);
+    const size_t blocks = (hc.groups + kWarpBlock / 32 - 1) / (kWarpBlock / 32);
     const unsigned grid = (unsigned)std::max<size_t>(1, blocks);
     const int tt = m.use_l1_norm ? kTransNone : use_x_star ? kTransThreshold : kTransSqrt;
     auto launch = [&](auto kernel) { kernel<<<grid, kWarpBlock, 0, stream>>>(ta); };
@@ -1061,13 +1132,7 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* b
                                             best);
   PPF_CUDA(cudaGetLastError());
   ctx.launches += 3;
-  float h[20];
-  PPF_CUDA(cudaMemcpyAsync(h, best, sizeof(h), cudaMemcpyDeviceToHost, stream));
-  PPF_CUDA(cudaStreamSynchronize(stream));
-  *best_score = h[16];
-  unsigned long long idx;
-  memcpy(&idx, h + 18, sizeof(idx));
-  return (size_t)idx;
+  return finish();
 }
 
 }  // namespace ppf

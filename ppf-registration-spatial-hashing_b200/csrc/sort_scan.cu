@@ -332,9 +332,8 @@ __global__ void __launch_bounds__(kRunThreads) runs_count(const uint32_t* __rest
   if (threadIdx.x == 0) tile_heads[blockIdx.x] = total;
 }
 
-// Exclusive scan of the per-tile head counts by one block (serial chunks).
-__global__ void __launch_bounds__(kRunThreads) runs_scan_tiles(uint32_t* __restrict__ v, size_t m,
-                                                               uint32_t* __restrict__ total_out) {
+// Exclusive scan of m values by one block (serial chunks).
+__device__ __forceinline__ void scan_chunks(uint32_t* __restrict__ v, size_t m, uint32_t* __restrict__ total_out) {
   __shared__ uint32_t s_scan[kRunWarps];
   __shared__ uint32_t s_carry;
   if (threadIdx.x == 0) s_carry = 0;
@@ -350,6 +349,49 @@ __global__ void __launch_bounds__(kRunThreads) runs_scan_tiles(uint32_t* __restr
     __syncthreads();
   }
   if (threadIdx.x == 0) *total_out = s_carry;
+}
+
+__global__ void __launch_bounds__(kRunThreads) runs_scan_tiles(uint32_t* __restrict__ v, size_t m,
+                                                               uint32_t* __restrict__ total_out) {
+  scan_chunks(v, m, total_out);
+}
+
+__global__ void __launch_bounds__(kRunThreads) scan_small(uint32_t* __restrict__ a, uint32_t* __restrict__ b, size_t n,
+                                                          const uint32_t* __restrict__ n_dev,
+                                                          uint32_t* __restrict__ total_out) {
+  scan_chunks(blockIdx.x ? b : a, n_dev ? min(n, (size_t)*n_dev) : n, total_out + blockIdx.x);
+}
+
+// Run table of at most kRunsSmall keys by one block, 8 keys per thread.
+constexpr int kRunsSmallThreads = 1024;
+constexpr uint32_t kRunsSmallItems = kRunsSmall / kRunsSmallThreads;
+__global__ void __launch_bounds__(kRunsSmallThreads) runs_small(const uint32_t* __restrict__ k, uint32_t n,
+                                                                uint32_t* __restrict__ uniq,
+                                                                uint32_t* __restrict__ first,
+                                                                uint32_t* __restrict__ count,
+                                                                uint32_t* __restrict__ k_out) {
+  __shared__ uint32_t s_scan[kRunsSmallThreads / 32];
+  __shared__ uint32_t s_first[kRunsSmall + 1];
+  const uint32_t base = threadIdx.x * kRunsSmallItems;
+  uint32_t heads = 0;
+  for (uint32_t i = 0; i < kRunsSmallItems; ++i) {
+    const uint32_t p = base + i;
+    if (p < n && (p == 0 || k[p] != k[p - 1])) heads |= 1u << i;
+  }
+  uint32_t total;
+  uint32_t r = block_excl_scan<kRunsSmallThreads / 32>(__popc(heads), s_scan, &total);
+  for (; heads; heads &= heads - 1) s_first[r++] = base + __ffs(heads) - 1;
+  if (threadIdx.x == 0) {
+    s_first[total] = n;
+    *k_out = total;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < total; i += kRunsSmallThreads) {
+    const uint32_t f = s_first[i];
+    uniq[i] = k[f];
+    first[i] = f;
+    count[i] = s_first[i + 1] - f;
+  }
 }
 
 __global__ void __launch_bounds__(kRunThreads) runs_emit(const uint32_t* __restrict__ k, size_t n,
@@ -467,8 +509,16 @@ void RadixSorter<K>::sort(K* keys, uint32_t* vals, bool vals_iota, size_t n, int
 template class RadixSorter<uint32_t>;
 template class RadixSorter<unsigned long long>;
 
-void exclusive_scan_small(uint32_t* v, size_t n, uint32_t* total_dev, cudaStream_t st) {
-  runs_scan_tiles<<<1, kRunThreads, 0, st>>>(v, n, total_dev);
+void exclusive_scan_small(uint32_t* a, uint32_t* b, size_t n, const uint32_t* n_dev, uint32_t* total_dev,
+                          cudaStream_t st) {
+  scan_small<<<b ? 2 : 1, kRunThreads, 0, st>>>(a, b, n, n_dev, total_dev);
+  PPF_CUDA(cudaGetLastError());
+}
+
+void build_runs_small(const uint32_t* sorted_keys, size_t n, uint32_t* uniq, uint32_t* first, uint32_t* count,
+                      uint32_t* k_dev, cudaStream_t st) {
+  PPF_REQUIRE(n <= kRunsSmall, PPF_ERR_INTERNAL, "too many keys for one block");
+  runs_small<<<1, kRunsSmallThreads, 0, st>>>(sorted_keys, (uint32_t)n, uniq, first, count, k_dev);
   PPF_CUDA(cudaGetLastError());
 }
 

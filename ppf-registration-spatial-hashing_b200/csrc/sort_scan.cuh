@@ -57,8 +57,17 @@ size_t build_runs(const uint32_t* sorted_keys, size_t n, uint32_t* uniq, uint32_
 size_t build_runs(const uint32_t* sorted_keys, size_t n, DevBuf& uniq, DevBuf& first, DevBuf& count,
                   DevBuf& scratch, cudaStream_t st, size_t* launches);
 
-// In-place exclusive scan of n uint32 by one block (for per-run tables of at
-// most a few million entries); *total_dev receives the sum.
-void exclusive_scan_small(uint32_t* v, size_t n, uint32_t* total_dev, cudaStream_t st);
+// The same for at most kRunsSmall keys in one launch of one block, without a
+// wait: *k_dev receives K, and uniq/first/count have room for n entries.
+constexpr size_t kRunsSmall = 8192;
+void build_runs_small(const uint32_t* sorted_keys, size_t n, uint32_t* uniq, uint32_t* first, uint32_t* count,
+                      uint32_t* k_dev, cudaStream_t st);
+
+// In-place exclusive scans of a and b (b may be null), n uint32 each, by one
+// block per array (for per-run tables of at most a few million entries);
+// total_dev[0] and total_dev[1] receive the sums.  n_dev, if not null, holds
+// the number of entries (at most n).
+void exclusive_scan_small(uint32_t* a, uint32_t* b, size_t n, const uint32_t* n_dev, uint32_t* total_dev,
+                          cudaStream_t st);
 
 }  // namespace ppf

@@ -1508,9 +1508,15 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
   kernel<<<(unsigned)std::min<size_t>(n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
   PPF_CUDA(cudaGetLastError());
   ctx.launches++;
-  uint32_t h[16];
-  PPF_CUDA(cudaMemcpyAsync(h, ctx.counters.ptr, 64, cudaMemcpyDeviceToHost, stream));
-  PPF_CUDA(cudaStreamSynchronize(stream));
+  // counters, flags word and bad-index record, one wait for all
+  uint32_t* const h = ctx.host;
+  auto read_back = [&]() {
+    PPF_CUDA(cudaEventRecord(ctx.ev[1], stream));
+    PPF_CUDA(cudaMemcpyAsync(h, ctx.counters.ptr, 64, cudaMemcpyDeviceToHost, stream));
+    PPF_CUDA(cudaMemcpyAsync(h + 16, ctx.flags.ptr, 32 + 80, cudaMemcpyDeviceToHost, stream));
+    PPF_CUDA(cudaStreamSynchronize(stream));
+  };
+  read_back();
   if (h[3]) {
     // Items that did not fit: grow the buffer (keeping what was emitted) to
     // what every item asked for, then count those items again.
@@ -1540,20 +1546,13 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
     r.n_redo = h[3];
-    PPF_CUDA(cudaMemcpyAsync(h, ctx.counters.ptr, 64, cudaMemcpyDeviceToHost, stream));
-    PPF_CUDA(cudaStreamSynchronize(stream));
+    read_back();
     PPF_REQUIRE(h[3] == 0, PPF_ERR_INTERNAL, "vote candidates still do not fit");
   }
-  PPF_CUDA(cudaEventRecord(ctx.ev[1], stream));
-  PPF_CUDA(cudaEventSynchronize(ctx.ev[1]));
   {
-    // flags word and bad-index record in one read
-    unsigned long long rec[14];
-    PPF_CUDA(cudaMemcpyAsync(rec, ctx.flags.ptr, sizeof(rec), cudaMemcpyDeviceToHost, stream));
-    PPF_CUDA(cudaStreamSynchronize(stream));
-    const uint32_t f = (uint32_t)(rec[0] & 0xffffffffu);
-    if (f & kFlagBadIndex) {
-      const unsigned long long* bad = rec + 4;
+    if (h[16] & kFlagBadIndex) {
+      unsigned long long bad[10];
+      memcpy(bad, h + 16 + 8, sizeof(bad));
       std::string detail;
       for (int k = 3; k < 10; ++k)
         detail += " " + std::to_string(bad[k] >> 32) + ":" + std::to_string(bad[k] & 0xffffffffu);
@@ -1650,6 +1649,12 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
     ctx.launches++;
   }
   std::vector<uint32_t> h((n + 1) * 16);
+  unsigned long long rec[14];  // flags word and bad-index record
+  auto read_flags = [&]() {
+    PPF_CUDA(cudaEventRecord(ctx.ev[1], stream));
+    PPF_CUDA(cudaMemcpyAsync(ctx.host, ctx.flags.ptr, sizeof(rec), cudaMemcpyDeviceToHost, stream));
+  };
+  read_flags();
   PPF_CUDA(cudaMemcpyAsync(h.data(), cnt0, (n + 1) * 64, cudaMemcpyDeviceToHost, stream));
   PPF_CUDA(cudaStreamSynchronize(stream));
   // Requests whose cells did not all fit: grow their buffers (keeping what was
@@ -1684,16 +1689,13 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
     kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
     PPF_CUDA(cudaGetLastError());
     ctx.launches++;
+    read_flags();
     PPF_CUDA(cudaMemcpyAsync(hc, cnt0 + 16 * i, 64, cudaMemcpyDeviceToHost, stream));
     PPF_CUDA(cudaStreamSynchronize(stream));
     PPF_REQUIRE(hc[3] == 0, PPF_ERR_INTERNAL, "vote candidates still do not fit");
   }
-  PPF_CUDA(cudaEventRecord(ctx.ev[1], stream));
-  PPF_CUDA(cudaEventSynchronize(ctx.ev[1]));
   {
-    unsigned long long rec[14];
-    PPF_CUDA(cudaMemcpyAsync(rec, ctx.flags.ptr, sizeof(rec), cudaMemcpyDeviceToHost, stream));
-    PPF_CUDA(cudaStreamSynchronize(stream));
+    memcpy(rec, ctx.host, sizeof(rec));
     if ((uint32_t)(rec[0] & 0xffffffffu) & kFlagBadIndex)
       throw Error(PPF_ERR_INTERNAL, "vote kernel index out of range: site " + std::to_string(rec[4]) +
                                         " value " + std::to_string(rec[5]) + " bound " + std::to_string(rec[6]));
