@@ -237,11 +237,14 @@ constexpr uint32_t kOffSlotKey = kOffEvK + kEvents;      // run | kExactGroup
 constexpr uint32_t kOffSlotCnt = kOffSlotKey + kSlots;   // events, then offset of the group
 constexpr uint32_t kOffPcRun = kOffSlotCnt + kSlots;     // piece: its run
 constexpr uint32_t kOffPcInf = kOffPcRun + kMaxPieces;   // piece: see piece_info
-constexpr uint32_t kOffFlags = kOffPcInf + kMaxPieces;   // per warp: flagged events
-constexpr uint32_t kOffAcc = (kOffFlags + kVoteWarps * 8 + 31) / 32 * 32;  // counters, see kRowStride
+// per warp: (block of the unit << 16 | event of the piece) pairs that hold
+// ambiguous votes
+constexpr uint32_t kNotesLen = 32;
+constexpr uint32_t kOffNotes = kOffPcInf + kMaxPieces;
+constexpr uint32_t kOffAcc = (kOffNotes + kVoteWarps * kNotesLen + 31) / 32 * 32;  // counters, see kRowStride
 // over the pieces while the list is filled: per warp the scene pairs that
 // await their lookup
-constexpr uint32_t kNearLen = 64;
+constexpr uint32_t kNearLen = 96;
 constexpr uint32_t kOffNear = kOffPcRun;
 static_assert(kVoteWarps * kNearLen <= 2 * kMaxPieces, "the waiting pairs fit the pieces");
 // over the event slot words once the list is grouped: the pieces' entries in
@@ -255,8 +258,6 @@ constexpr uint32_t kOffPcInc = kOffPcUnit + kMaxPieces + 1;
 constexpr uint32_t kTabWords = 60, kQueueLen = 32;
 constexpr uint32_t kOffTab = kOffSlotKey;
 constexpr uint32_t kOffQueue = kOffTab + kVoteWarps * kTabWords;
-// events of a swept piece with ambiguous votes in the current block, a bit each
-constexpr uint32_t kFlagWords = (kPieceEvents + 31) / 32;
 static_assert(kVoteWarps * (kTabWords + 2 * kQueueLen) <= 2 * kSlots, "tables and queues fit the slots");
 
 // Accumulator: plane j holds the 16-bit counters of bins (2j, 2j + 1) of every
@@ -332,8 +333,7 @@ extern __shared__ __align__(16) uint32_t smem[];
 
 // The warp's histogram table and queue.
 __device__ __forceinline__ uint32_t* warp_tab() { return smem + kOffTab + (threadIdx.x >> 5) * kTabWords; }
-static_assert(kFlagWords <= 8, "flag words per warp");
-__device__ __forceinline__ uint32_t* warp_flags() { return smem + kOffFlags + (threadIdx.x >> 5) * 8; }
+__device__ __forceinline__ uint32_t* warp_notes() { return smem + kOffNotes + (threadIdx.x >> 5) * kNotesLen; }
 __device__ __forceinline__ uint32_t* warp_queue() { return smem + kOffQueue + (threadIdx.x >> 5) * 2 * kQueueLen; }
 
 __device__ __forceinline__ uint32_t wrap30(int b) { return (uint32_t)(b < 0 ? b + PPF_N_ANGLE : b); }
@@ -429,37 +429,39 @@ __device__ __forceinline__ uint32_t queue_votes(const VoteArgs& a, const VoteSha
   return qn;
 }
 
-// Queues the ambiguous votes of a block's flagged events (a bit each) and
-// clears the flags; returns the queue's length and the lane's ambiguous votes.
-// Out of line and called at a block's end, where its callers hold little in
-// registers: inside their loops it spilled a fifth of the sweep's accesses.
+// Queues the ambiguous votes of the noted (block, event) pairs of a unit;
+// returns the queue's length and the lane's ambiguous votes.  Notes past the
+// array's end were not stored: the block that made them, `blk`, whose notes
+// start at `own`, is then searched with all events of the piece.  Out of line
+// and called about once per 24 notes at a block's end, where its callers hold
+// little in registers: inside their loops it spilled a fifth of the sweep's
+// shared-memory accesses, and called once per block it still saved and
+// restored 6% of them.
 template <bool kCheck>
-__device__ __noinline__ uint2 queue_flagged(const VoteArgs& a, const VoteShared& sh, uint32_t pos, uint32_t end,
-                                            uint32_t ev0, bool sweep, uint32_t qn) {
-  uint32_t* const flags = warp_flags();
+__device__ __noinline__ uint2 queue_noted(const VoteArgs& a, const VoteShared& sh, uint32_t start, uint32_t end,
+                                          uint32_t ev0, uint32_t cnt, uint32_t n_notes, uint32_t own, uint32_t blk,
+                                          bool sweep, uint32_t qn) {
+  const uint32_t* const notes = warp_notes();
   uint32_t n_exact = 0;
   __syncwarp();
+  const bool over = n_notes > kNotesLen;
+  const uint32_t n = over ? own + cnt : n_notes;
 #pragma unroll 1
-  for (uint32_t wd = 0; wd < kFlagWords; ++wd) {
-    uint32_t left = flags[wd];
-    while (left) {
-      const uint32_t ev = ev0 + 32 * wd + __ffs(left) - 1;
-      left &= left - 1;
-      const uint32_t re = smem[kOffEvW + ev] & (kTurn - 1u);
-      uint32_t amb = 0;
+  for (uint32_t j = 0; j < n; ++j) {
+    const uint32_t note = over && j >= own ? blk << 16 | (j - own) : notes[j];
+    const uint32_t pos = start + (note >> 16) * kBlock, ev = ev0 + (note & 0xffffu);
+    const uint32_t re = smem[kOffEvW + ev] & (kTurn - 1u);
+    uint32_t amb = 0;
 #pragma unroll
-      for (int k = 0; k < kPerLane; ++k) {
-        const uint32_t p = pos + 32u * k + (threadIdx.x & 31);
-        if (p < end && in_range<kCheck>(a, 28, p, a.P)) {
-          const uint32_t r = ((__ldg(a.entries + p) & (kTurn - 1u)) * PPF_N_ANGLE) & (kTurn - 1u);
-          if (((re - r + kMargin - 1u) & (kTurn - 1u)) < 2 * kMargin - 1) amb |= 1u << k;
-        }
+    for (int k = 0; k < kPerLane; ++k) {
+      const uint32_t p = pos + 32u * k + (threadIdx.x & 31);
+      if (p < end && in_range<kCheck>(a, 28, p, a.P)) {
+        const uint32_t r = ((__ldg(a.entries + p) & (kTurn - 1u)) * PPF_N_ANGLE) & (kTurn - 1u);
+        if (((re - r + kMargin - 1u) & (kTurn - 1u)) < 2 * kMargin - 1) amb |= 1u << k;
       }
-      n_exact += __popc(amb);
-      qn = queue_votes<kCheck>(a, sh, amb, pos, ev, sweep, qn);
     }
-    __syncwarp();
-    flags[wd] = 0u;
+    n_exact += __popc(amb);
+    qn = queue_votes<kCheck>(a, sh, amb, pos, ev, sweep, qn);
   }
   __syncwarp();
   return make_uint2(qn, n_exact);
@@ -500,7 +502,8 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
   const uint32_t* const ev = smem + kOffEvW + ev0;
   uint32_t* const acc = smem + kOffAcc;
   uint32_t* const tab = warp_tab();
-  uint32_t* const flags = warp_flags();  // (all clear between units)
+  uint32_t* const notes = warp_notes();
+  uint32_t n_notes = 0;
   const uint32_t rs = a.r_shift;
   const uint32_t* const entries = a.entries;  // (a copy: a's fields are read anew after every atomic)
   uint32_t passed = 0;  // events of a bucket below the block's first: counted in H as Q_s - 1
@@ -585,7 +588,7 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
     // events among the block's entries, and within the margin of one; a block
     // near R = 0 meets the margin across it and looks at every event
     const bool edge = rmin < kMargin || rmax > kTurn - kMargin;
-    bool flagged = false;
+    const uint32_t own_notes = n_notes;
     for (uint32_t q = edge ? 0u : min(passed, done); q < cnt; ++q) {
       const uint32_t w = ev[q], re = w & (kTurn - 1u), qe = w >> PPF_ANGLE_BITS;
       if (!edge && (re >> rs) > b1 && re >= rmax + kMargin) break;
@@ -605,15 +608,16 @@ __device__ __noinline__ uint2 sweep_unit(const VoteArgs& a, const VoteShared& sh
         }
       }
       if (__any_sync(0xffffffffu, nearest < 2 * kMargin - 1)) {
-        flags[q >> 5] |= 1u << (q & 31);  // (all lanes write the same word)
-        flagged = true;
-        __syncwarp();
+        if (n_notes < kNotesLen) notes[n_notes] = (pos - start) / kBlock << 16 | q;  // (by all lanes alike)
+        ++n_notes;
       }
     }
-    if (flagged) {
-      const uint2 r = queue_flagged<kCheck>(a, sh, pos, end, ev0, true, qn);
+    if (n_notes > kNotesLen - 8 || (n_notes && pos + kBlock >= end)) {
+      const uint2 r = queue_noted<kCheck>(a, sh, start, end, ev0, cnt, n_notes, own_notes, (pos - start) / kBlock, true,
+                                          qn);
       qn = r.x;
       n_exact += r.y;
+      n_notes = 0;
     }
   }
   return make_uint2(qn, n_exact);
@@ -634,12 +638,13 @@ __device__ __noinline__ uint2 count_unit(const VoteArgs& a, const VoteShared& sh
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t* const entries = a.entries;
   uint32_t* const acc = smem + kOffAcc;
-  uint32_t* const flags = warp_flags();
+  uint32_t* const notes = warp_notes();
+  uint32_t n_notes = 0;
   for (uint32_t pos = start; pos < end; pos += kBlock) {
     const uint32_t n = min((uint32_t)kBlock, end - pos);
     uint32_t c[kPerLane];
     load_block(entries, pos, end, c);
-    bool flagged = false;
+    const uint32_t own_notes = n_notes;
     for (uint32_t g = 0; g < cnt; ++g) {
       const uint32_t base = count_angle(smem[kOffEvW + ev0 + g], 0u);
       bool amb = false;  // (a lane past the end may say so too)
@@ -653,15 +658,16 @@ __device__ __noinline__ uint2 count_unit(const VoteArgs& a, const VoteShared& sh
         }
       }
       if (__any_sync(0xffffffffu, amb)) {
-        flags[g >> 5] |= 1u << (g & 31);
-        flagged = true;
-        __syncwarp();
+        if (n_notes < kNotesLen) notes[n_notes] = (pos - start) / kBlock << 16 | g;
+        ++n_notes;
       }
     }
-    if (flagged) {
-      const uint2 r = queue_flagged<kCheck>(a, sh, pos, end, ev0, false, qn);
+    if (n_notes > kNotesLen - 8 || (n_notes && pos + kBlock >= end)) {
+      const uint2 r = queue_noted<kCheck>(a, sh, start, end, ev0, cnt, n_notes, own_notes, (pos - start) / kBlock,
+                                          false, qn);
       qn = r.x;
       n_exact += r.y;
+      n_notes = 0;
     }
   }
   return make_uint2(qn, n_exact);
@@ -686,16 +692,19 @@ __device__ __noinline__ void exact_unit(const VoteArgs& a, const VoteShared& sh,
   }
 }
 
-// A warp's place in the walk over the scene: its next 32 points and the pairs
-// of its buffer that still await their lookup.
+// A warp's place in the walk over the scene: its next points and the pairs of
+// its buffer that still await their lookup.
+constexpr uint32_t kWalkStep = 2 * kVoteThreads;
+static_assert(31 + 64 <= kNearLen && kNearLen == 3 * 32, "a step's pairs fit behind the waiting ones");
 struct WalkState {
   uint32_t base = 0, n_near = 0;
+  uint32_t waiting[3];  // the waiting pairs, 32 k + lane, while the buffer is in other use
 };
 
 // Fills the list with the events of s_r from the warps' places on, until the
 // scene ends (false) or the list is full (true; uniform over the block).
 //
-// Warp w takes points 32 w + lane of every 1024.  With the model's feature
+// Warp w takes points 32 w + lane of every 1024, two such steps at a time.  With the model's feature
 // table it first looks only at the distance: a pair whose distance row has no
 // run is dropped, the others wait in the warp's buffer until there are 32, so
 // that the angles (three acosf), the table lookup and the frame angle run on
@@ -709,8 +718,9 @@ __device__ __forceinline__ bool walk_scene(const VoteArgs& a, uint32_t sr, bool 
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* const near = smem + kOffNear + warp * kNearLen;
   // (the buffers lie over the pieces, which the list's votes have read)
-  __shared__ uint32_t s_near[kVoteWarps][32];
-  if (ws.n_near && lane < ws.n_near) near[lane] = s_near[warp][lane];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (32u * k + lane < ws.n_near) near[32 * k + lane] = ws.waiting[k];
   for (uint32_t i = tid; i < kSlots; i += kVoteThreads) {
     slot_key[i] = kNoRun;
     slot_cnt[i] = 0u;
@@ -724,23 +734,32 @@ __device__ __forceinline__ bool walk_scene(const VoteArgs& a, uint32_t sr, bool 
   for (;;) {
     // gather pairs until 32 wait or the scene ends
     while (ws.n_near < 32 && ws.base < a.n_s) {
-      const uint32_t i = ws.base + tid;
-      bool keep = i < a.n_s && i != sr;
-      if (keep && a.lut) {
-        const float4 q = a.s_pts[i];
-        const float3 d = make_float3(q.x - pr.x, q.y - pr.y, q.z - pr.z);
-        const float len = norm3(d);
-        // rows past the flags are looked up by key
-        keep = !isnan(len);
-        if (len < (float)(kFlagRows - 1) * a.d_dist) {
-          const uint32_t nd = (uint32_t)quant_index(len, a.d_dist, inv_d);
-          keep = sh.rows[nd / 32] >> (nd % 32) & 1u;
-        }
+      // two points per lane, so that two loads are in flight
+      bool keep[2];
+      float4 q[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t i = ws.base + kVoteThreads * k + tid;
+        keep[k] = i < a.n_s && i != sr;
+        if (keep[k] && a.lut) q[k] = a.s_pts[i];
       }
-      const uint32_t in = __ballot_sync(0xffffffffu, keep);
-      if (keep) near[ws.n_near + __popc(in & ((1u << lane) - 1u))] = i;
-      ws.n_near += __popc(in);
-      ws.base += kVoteThreads;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (keep[k] && a.lut) {
+          const float3 d = make_float3(q[k].x - pr.x, q[k].y - pr.y, q[k].z - pr.z);
+          const float len = norm3(d);
+          // rows past the flags are looked up by key
+          keep[k] = !isnan(len);
+          if (len < (float)(kFlagRows - 1) * a.d_dist) {
+            const uint32_t nd = (uint32_t)quant_index(len, a.d_dist, inv_d);
+            keep[k] = sh.rows[nd / 32] >> (nd % 32) & 1u;
+          }
+        }
+        const uint32_t in = __ballot_sync(0xffffffffu, keep[k]);
+        if (keep[k]) near[ws.n_near + __popc(in & ((1u << lane) - 1u))] = ws.base + kVoteThreads * k + tid;
+        ws.n_near += __popc(in);
+      }
+      ws.base += kWalkStep;
     }
     __syncwarp();
     const uint32_t n = min(ws.n_near, 32u);
@@ -827,71 +846,106 @@ __device__ __forceinline__ bool walk_scene(const VoteArgs& a, uint32_t sr, bool 
         }
       }
     }
-    // the buffer's rest (at most 31 pairs) moves to its front
+    // the buffer's rest (at most 63 pairs) moves to its front
     __syncwarp();
     const uint32_t rest = ws.n_near - n;
-    const uint32_t moved = lane < rest ? near[n + lane] : 0u;
+    const uint32_t m0 = lane < rest ? near[n + lane] : 0u, m1 = lane + 32 < rest ? near[n + lane + 32] : 0u;
     __syncwarp();
-    if (lane < rest) near[lane] = moved;
+    if (lane < rest) near[lane] = m0;
+    if (lane + 32 < rest) near[lane + 32] = m1;
     ws.n_near = rest;
     __syncwarp();
   }
   // what waits is kept aside while the list's pieces take the buffers' place
-  // (at most 32 + 31 pairs; those past 32 are walked again)
   __syncwarp();
-  if (ws.n_near > 32) {
-    // the last step's points start over: nothing of them was looked up
-    const uint32_t first = ws.base - kVoteThreads;
-    ws.n_near = __popc(__ballot_sync(0xffffffffu, near[lane] < first + warp * 32));
-    ws.base = first;
-  }
-  if (lane < ws.n_near) s_near[warp][lane] = near[lane];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) ws.waiting[k] = 32u * k + lane < ws.n_near ? near[32 * k + lane] : 0u;
   __syncwarp();
   return __syncthreads_or(full);
 }
 
-// Sorts a swept piece's events by R (rank by comparison: at most 255 events)
-// and returns an upper bound of how many of them one entry can vote into one
-// bin: its votes for a bin come from one bin's width of event angles, plus
-// the margin on both sides for votes near an edge, which lies within four
-// neighbouring half bins.
+// Ascending bitonic sort of 32 M distinct words over a warp; word 32 m + lane
+// is x[m] of the lane.
+template <int M>
+__device__ __forceinline__ void warp_sort(uint32_t (&x)[M]) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 2; k <= 32 * M; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j >= 32; j >>= 1) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int o = m ^ (j >> 5);
+        if (o > m) {
+          const uint32_t lo = min(x[m], x[o]), hi = max(x[m], x[o]);
+          const bool up = ((32 * m) & k) == 0;  // k > 32: the same for all lanes
+          x[m] = up ? lo : hi;
+          x[o] = up ? hi : lo;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = k >> 1 < 16 ? k >> 1 : 16; j > 0; j >>= 1) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x[m], j);
+        const bool up = (((uint32_t)(32 * m) | lane) & (uint32_t)k) == 0, low = (lane & (uint32_t)j) == 0;
+        x[m] = up == low ? min(x[m], y) : max(x[m], y);
+      }
+    }
+  }
+}
+
+// The sort of sort_piece for pieces of at most 32 M events: R above the
+// event's index, so that the words are distinct and carry their events.
+template <int M>
+__device__ __forceinline__ void order_events(uint32_t* ew, uint32_t* ei, uint32_t cnt) {
+  static_assert(32 * M <= 256, "an index byte below the 21 bits of R");
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t x[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const uint32_t j = 32u * m + lane;
+    x[m] = j < cnt ? (ew[j] & (kTurn - 1u)) << 8 | j : 0xffffff00u | j;
+  }
+  warp_sort<M>(x);
+  uint32_t w[M], i[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const uint32_t from = x[m] & 0xffu;
+    w[m] = from < cnt ? ew[from] : 0u;
+    i[m] = from < cnt ? ei[from] : 0u;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const uint32_t j = 32u * m + lane;
+    if (j < cnt) {
+      ew[j] = w[m];
+      ei[j] = i[m];
+    }
+  }
+}
+
+// Sorts a swept piece's events by R and returns an upper bound of how many of
+// them one entry can vote into one bin: its votes for a bin come from one
+// bin's width of event angles, plus the margin on both sides for votes near an
+// edge, which lies within four neighbouring half bins.
 __device__ __forceinline__ uint32_t sort_piece(uint32_t ev0, uint32_t cnt) {
   uint32_t* const tab = warp_tab();
   const uint32_t lane = threadIdx.x & 31;
-  constexpr int kPer = (kPieceEvents + 31) / 32;
   uint32_t* const ew = smem + kOffEvW + ev0;
   uint32_t* const ei = smem + kOffEvI + ev0;
-  uint32_t w[kPer], pi[kPer], rank[kPer];
   constexpr uint32_t kHalves = 2 * PPF_N_ANGLE;
   static_assert(kHalves <= kTabWords, "a counter per half bin");
   for (uint32_t k = lane; k < kHalves; k += 32) tab[k] = 0u;
   __syncwarp();
-#pragma unroll
-  for (int m = 0; m < kPer; ++m) {
-    const uint32_t j = 32u * m + lane;
-    w[m] = j < cnt ? ew[j] : 0u;
-    pi[m] = j < cnt ? ei[j] : 0u;
-    rank[m] = 0;
-    if (j < cnt) atomicAdd(tab + (w[m] >> (PPF_ANGLE_BITS - 1)), 1u);
-  }
-  for (uint32_t q = 0; q < cnt; ++q) {
-    const uint32_t r = ew[q] & (kTurn - 1u);
-#pragma unroll
-    for (int m = 0; m < kPer; ++m) {
-      if (32u * m < cnt) {
-        const uint32_t own = w[m] & (kTurn - 1u);
-        rank[m] += (r < own || (r == own && q < 32u * m + lane)) ? 1u : 0u;
-      }
-    }
-  }
+  for (uint32_t j = lane; j < cnt; j += 32) atomicAdd(tab + (ew[j] >> (PPF_ANGLE_BITS - 1)), 1u);
+  if (cnt <= 32) order_events<1>(ew, ei, cnt);
+  else if (cnt <= 64) order_events<2>(ew, ei, cnt);
+  else if (cnt <= 128) order_events<4>(ew, ei, cnt);
+  else order_events<8>(ew, ei, cnt);
   __syncwarp();
-#pragma unroll
-  for (int m = 0; m < kPer; ++m) {
-    if (32u * m + lane < cnt) {
-      ew[rank[m]] = w[m];
-      ei[rank[m]] = pi[m];
-    }
-  }
   uint32_t win = 0;
   for (uint32_t k = lane; k < kHalves; k += 32) {
     uint32_t four = 0;
@@ -991,7 +1045,6 @@ __device__ __forceinline__ void vote_units(const VoteArgs& a, VoteShared& sh, Vo
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t* const pc_unit = smem + kOffPcUnit;
   if (tid == 0) sh.next = u0 + kVoteWarps;
-  if (lane < 8) warp_flags()[lane] = 0u;
   block_sync();
   uint32_t qn = 0;
   const uint32_t stride = (n_pieces + 31) / 32;
