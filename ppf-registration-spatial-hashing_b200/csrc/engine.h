@@ -82,7 +82,7 @@ struct ModelTables {
   DevBuf weights;        // float vote weights (default 1)
   // all ordered pairs, sorted by feature key (stable: pair index order)
   size_t P = 0;
-  DevBuf keys;           // uint32 sorted keys
+  DevBuf keys;           // uint32 run of each pair in map order (kept for the self-checks only)
   DevBuf pairs;          // uint32 pair index r*n + i (the hash array's data map)
   // Vote order: by run, then chunk of m_r, then buckets of 2^r_shift of
   // R = 30 x angle mod 2^21 (the angle's position inside an alpha bin), each

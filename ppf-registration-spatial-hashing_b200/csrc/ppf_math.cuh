@@ -78,7 +78,14 @@ __device__ __forceinline__ float dot3(float3 a, float3 b) {
 __device__ __forceinline__ float dot4(float4 a, float4 b) {
   return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
 }
-__device__ __forceinline__ float norm3(float3 a) { return sqrtf(dot3(a, a)); }
+// The dot product of the pair features with its contraction written out (y y'
+// rounded, x x' fused onto it, then z z'), as the reference's kernels round
+// it: left to the compiler, the kernel around it decides which product is
+// fused, and one in 1e5 features changes.
+__device__ __forceinline__ float dot3_pair(float3 a, float3 b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float norm3(float3 a) { return sqrtf(dot3_pair(a, a)); }
 __device__ __forceinline__ float norm4(float4 a) { return sqrtf(dot4(a, a)); }
 
 // x rounded down to a multiple of y, as x - fmodf(x, y) (src/cuda/kernel.cu:90-92).
@@ -108,9 +115,9 @@ __device__ __forceinline__ float4 pair_feature(float3 p1, float3 n1, float3 p2, 
   d.z = p2.z - p1.z;
   float4 f;
   f.x = norm3(d);
-  f.y = acosf(dot3(n1, d) / (norm3(n1) * norm3(d)));
-  f.z = acosf(dot3(n2, d) / (norm3(n2) * norm3(d)));
-  f.w = acosf(dot3(n1, n2) / (norm3(n1) * norm3(n2)));
+  f.y = acosf(dot3_pair(n1, d) / (norm3(n1) * norm3(d)));
+  f.z = acosf(dot3_pair(n2, d) / (norm3(n2) * norm3(d)));
+  f.w = acosf(dot3_pair(n1, n2) / (norm3(n1) * norm3(n2)));
   f.x = quant_down(f.x, d_dist);
   f.y = quant_down(f.y, PPF_D_ANGLE);
   f.z = quant_down(f.z, PPF_D_ANGLE);
@@ -135,9 +142,9 @@ __device__ __forceinline__ uint32_t angle_index(float angle) {
 
 // Index of the three angles of pair_feature, d = p2 - p1 and |d| given.
 __device__ __forceinline__ uint32_t pair_angles(float3 n1, float3 n2, float3 d, float len) {
-  const uint32_t y = angle_index(acosf(dot3(n1, d) / (norm3(n1) * len)));
-  const uint32_t z = angle_index(acosf(dot3(n2, d) / (norm3(n2) * len)));
-  const uint32_t w = angle_index(acosf(dot3(n1, n2) / (norm3(n1) * norm3(n2))));
+  const uint32_t y = angle_index(acosf(dot3_pair(n1, d) / (norm3(n1) * len)));
+  const uint32_t z = angle_index(acosf(dot3_pair(n2, d) / (norm3(n2) * len)));
+  const uint32_t w = angle_index(acosf(dot3_pair(n1, n2) / (norm3(n1) * norm3(n2))));
   return (y * kAngleValues + z) * kAngleValues + w;
 }
 

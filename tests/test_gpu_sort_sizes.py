@@ -16,7 +16,8 @@ def test_hash_array_is_the_stable_sort_of_the_keys(pkg, ctx, n):
     p = rng.uniform(-0.05, 0.05, (n, 3)).astype(np.float32)
     q = rng.normal(size=(n, 3)).astype(np.float32)
     q /= np.linalg.norm(q, axis=1, keepdims=True)
-    for d in (0.02, 0.5):  # many runs, few runs
+    # many runs, few runs, and pairs past the feature table (the runs then come from sorted keys)
+    for d in (0.02, 0.5, 0.0006):
         keys = pkg.pair_keys((p, q), d, 1, context=ctx).ravel()
         order = np.argsort(keys, kind="stable").astype(np.uint32)
         uniq, first, count = np.unique(keys, return_index=True, return_counts=True)
