@@ -131,7 +131,6 @@ struct LookupState {
   DevBuf trans0;      // float U*3 (before clustering)
   DevBuf quats;       // float U*4
   DevBuf cell_keys;   // uint32 U
-  DevBuf adj;         // uint32 U*27
   DevBuf scores;      // float U
   DevBuf cells_sorted, cells_map, cells_uniq, cells_first, cells_count;
   DevBuf cells3;      // int4 U: integer cell of each pose

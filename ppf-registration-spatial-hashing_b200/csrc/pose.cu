@@ -144,7 +144,6 @@ struct PoseArgs {
   float* weighted;
   uint32_t* cell_keys;
   uint32_t* cells_sorted;  // cell_keys again, to be sorted
-  uint32_t* adj;
   int4* cells3;
 };
 
@@ -187,12 +186,6 @@ __global__ void poses_kernel(PoseArgs a) {
     a.cell_keys[i] = key;
     a.cells_sorted[i] = key;
     a.cells3[i] = make_int4(c.x, c.y, c.z, 0);
-    uint32_t* adj = a.adj + 27 * i;
-    int idx = 0;
-    for (int di = -1; di < 2; ++di)
-      for (int dj = -1; dj < 2; ++dj)
-        for (int dk = -1; dk < 2; ++dk, ++idx)
-          adj[idx] = (di == 0 && dj == 0 && dk == 0) ? 0u : cell_key(c.x + di, c.y + dj, c.z + dk);
   }
 }
 
@@ -201,7 +194,7 @@ struct ClusterArgs {
   const float* trans0;
   const float* quats;
   const float* weighted;
-  const uint32_t* adj;
+  const int4* cells3;
   const uint32_t* uniq;
   const uint32_t* first;
   const uint32_t* count;
@@ -224,8 +217,10 @@ __global__ void cluster_kernel(ClusterArgs a) {
     float4 q = make_float4(a.quats[4 * i], a.quats[4 * i + 1], a.quats[4 * i + 2], a.quats[4 * i + 3]);
     float c = 1;
     float3 to = t;
+    const int4 cell = a.cells3[i];
     for (int b = 0; b < 27; ++b) {
-      uint32_t key = a.adj[27 * i + b];
+      if (b == 13) continue;  // the pose's own cell
+      const uint32_t key = cell_key(cell.x + b / 9 - 1, cell.y + b / 3 % 3 - 1, cell.z + b % 3 - 1);
       if (key == 0u) continue;
       size_t lo = 0, hi = a.Kc;
       while (lo < hi) {
@@ -926,7 +921,6 @@ void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState
   a.weighted = grow<float>(st.weighted, U);
   a.cell_keys = grow<uint32_t>(st.cell_keys, U);
   a.cells_sorted = grow<uint32_t>(st.cells_sorted, U);
-  a.adj = grow<uint32_t>(st.adj, U * 27);
   a.cells3 = grow<int4>(st.cells3, U);
   grow<float>(st.trans, U * 3);
   grow<float>(st.scores, U);
@@ -1003,7 +997,7 @@ size_t cluster_poses_gpu(Context& ctx, const Model& m, LookupState& st, float* p
   a.trans0 = st.trans0.as<float>();
   a.quats = st.quats.as<float>();
   a.weighted = st.weighted.as<float>();
-  a.adj = st.adj.as<uint32_t>();
+  a.cells3 = st.cells3.as<int4>();
   a.uniq = uq;
   a.first = fi;
   a.count = ct;
