@@ -100,7 +100,8 @@ struct VoteArgs {
   uint32_t* cand_count;
   uint32_t* n_cand;
   uint32_t cand_cap;
-  unsigned long long* n_needed;  // cells all items asked to emit
+  unsigned long long* n_needed;  // cells all items of the launch asked to emit
+  uint32_t cand_base;            // cells already in the buffer when the launch began
   uint32_t* redo_items;          // items that did not fit the buffer
   uint32_t* n_redo;
   uint32_t n_items_total;        // capacity of redo_items
@@ -303,20 +304,6 @@ struct VoteStats {
   unsigned long long votes = 0, matched = 0, exact = 0;
 };
 
-__device__ __forceinline__ void flush_stats(const VoteArgs& a, VoteStats& st) {
-  for (int o = 16; o; o >>= 1) {
-    st.votes += __shfl_xor_sync(0xffffffffu, st.votes, o);
-    st.matched += __shfl_xor_sync(0xffffffffu, st.matched, o);
-    st.exact += __shfl_xor_sync(0xffffffffu, st.exact, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (st.votes) atomicAdd(&a.stats[0], st.votes);
-    if (st.matched) atomicAdd(&a.stats[1], st.matched);
-    if (st.exact) atomicAdd(&a.stats[2], st.exact);
-  }
-  st = VoteStats();
-}
-
 // Fetches the next work item into sh.item (one atomic per block).
 __device__ __forceinline__ uint32_t fetch_item(uint32_t* work_counter, VoteShared& sh) {
   if ((threadIdx.x >> 5) == 0) {
@@ -330,6 +317,30 @@ __device__ __forceinline__ uint32_t fetch_item(uint32_t* work_counter, VoteShare
 }
 
 extern __shared__ __align__(16) uint32_t smem[];
+
+// Adds the block's statistics to the request's and clears them.  Called by the
+// whole block between items, through the words of the event list: one atomic
+// per counter and block.  (One per warp were 14000 on three addresses at the
+// end of a launch.)
+__device__ __forceinline__ void flush_stats(const VoteArgs& a, VoteStats& st) {
+  unsigned long long v[3] = {st.votes, st.matched, st.exact};
+  unsigned long long* const part = reinterpret_cast<unsigned long long*>(smem + kOffEvW);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(kVoteWarps == 32 && kEvents >= 3 * 32 * 2, "a lane per warp, in the event words");
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    for (int o = 16; o; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane == 0) part[32 * k + warp] = v[k];
+  }
+  block_sync();
+  if (warp < 3) {
+    unsigned long long t = part[32 * warp + lane];
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0 && t) atomicAdd(&a.stats[warp], t);
+  }
+  block_sync();
+  st = VoteStats();
+}
 
 // The warp's histogram table and queue.
 __device__ __forceinline__ uint32_t* warp_tab() { return smem + kOffTab + (threadIdx.x >> 5) * kTabWords; }
@@ -1245,36 +1256,27 @@ __device__ __forceinline__ void emit_chunk(const VoteArgs& a, uint32_t sr, uint3
   auto kept = [&](uint32_t cnt) { return cnt != 0u && (a.emit_all || (float)cnt > floor_v); };
   // All-or-nothing slot reservation for the chunk's cells: a chunk that does
   // not fit writes nothing and is queued for a second launch after the
-  // buffer has grown, so the buffer never holds a partial chunk.
+  // buffer has grown, so the buffer never holds a partial chunk.  Slots are
+  // what an atomic addition to the cells asked for returns: that total only
+  // grows, so the chunks that fit are the first ones added and lie without
+  // gaps, and n_cand is the sum of theirs.  (A compare-and-swap on n_cand took
+  // 34000 cycles where 140 blocks emitted at once, a quarter of a launch of
+  // one small item per block.)
   uint32_t my_n = 0;
   each([&](uint32_t, uint32_t, uint32_t cnt) { my_n += kept(cnt) ? 1u : 0u; });
   uint32_t item_total;
   const uint32_t my_off = block_excl_scan(my_n, sh.scan_emit, item_total);
   if (item_total == 0) return;  // uniform
-  if (warp == 0) {
-    // The whole warp walks the reservation loop in lockstep (lane 0 issues
-    // the atomics, every exit condition is warp-uniform).
-    uint32_t base_slot = 0xffffffffu;
-    if (lane == 0) atomicAdd(a.n_needed, (unsigned long long)item_total);
-    uint32_t old = 0;
-    if (lane == 0) old = *(volatile uint32_t*)a.n_cand;
-    old = __shfl_sync(0xffffffffu, old, 0);
-    for (int tries = 0; tries < (1 << 20); ++tries) {
-      if ((unsigned long long)old + item_total > a.cand_cap) break;
-      uint32_t prev = 0;
-      if (lane == 0) prev = atomicCAS(a.n_cand, old, old + item_total);
-      prev = __shfl_sync(0xffffffffu, prev, 0);
-      if (prev == old) {
-        base_slot = old;
-        break;
-      }
-      old = prev;
-    }
-    if (base_slot == 0xffffffffu && lane == 0) {
+  if (tid == 0) {
+    const unsigned long long at = a.cand_base + atomicAdd(a.n_needed, (unsigned long long)item_total);
+    const bool fits = at + item_total <= a.cand_cap;
+    if (fits) {
+      atomicAdd(a.n_cand, item_total);
+    } else {
       const uint32_t k = atomicAdd(a.n_redo, 1u);
       if (in_range<kCheck>(a, 9, k, a.n_items_total)) a.redo_items[k] = item;
     }
-    if (lane == 0) sh.base = base_slot;
+    sh.base = fits ? (uint32_t)at : 0xffffffffu;
   }
   block_sync();
   const uint32_t item_base = sh.base;
@@ -1530,7 +1532,8 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
   const uint32_t n_items = a.n_ref * a.n_cg;
   if (s.n < 2 || n_items == 0) return r;
   // counters: [0] work, [1] max, [2] n_cand, [3] n_redo, [4..9] 3 x u64 stats,
-  // [10..11] u64 n_needed, [12] work counter of the second launch
+  // [10..11] u64 n_needed, [12] work counter and [14..15] n_needed of the
+  // second launch
   ctx.counters.reserve(64);
   PPF_CUDA(cudaMemsetAsync(ctx.counters.ptr, 0, 64, stream));
   // flags word and the bad-index record at byte 32 (site, value, bound, 7 words of detail)
@@ -1594,6 +1597,8 @@ VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit
     a.item_list = items.as<uint32_t>();
     a.n_items = h[3];
     a.work_counter = cnt + 12;
+    a.n_needed = reinterpret_cast<unsigned long long*>(cnt + 14);
+    a.cand_base = h[2];
     PPF_CUDA(cudaMemsetAsync(a.n_redo, 0, 4, stream));
     kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
     PPF_CUDA(cudaGetLastError());
@@ -1632,8 +1637,8 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
   std::vector<VoteArgs> args(n);
   std::vector<uint32_t> item_off(n + 1, 0);
   // per request 16 counter words ([1] max, [2] n_cand, [3] n_redo, [4..9]
-  // stats, [10..11] n_needed, [12] work counter of its redo launch), then the
-  // batch's own work counter
+  // stats, [10..11] n_needed, [12] work counter and [14..15] n_needed of its
+  // redo launch), then the batch's own work counter
   ctx.batch_counters.reserve((n + 1) * 64);
   PPF_CUDA(cudaMemsetAsync(ctx.batch_counters.ptr, 0, (n + 1) * 64, stream));
   PPF_CUDA(cudaMemsetAsync(ctx.flags.ptr, 0, 32 + 80, stream));
@@ -1738,6 +1743,8 @@ void run_votes_batch(Context& ctx, std::vector<BatchVote>& reqs) {
     a.item_list = items.as<uint32_t>();
     a.n_items = hc[3];
     a.work_counter = cnt0 + 16 * i + 12;
+    a.n_needed = reinterpret_cast<unsigned long long*>(cnt0 + 16 * i + 14);
+    a.cand_base = hc[2];
     PPF_CUDA(cudaMemsetAsync(a.n_redo, 0, 4, stream));
     kernel<<<(unsigned)std::min<size_t>(a.n_items, (size_t)sm_count()), kVoteThreads, kVoteSmemBytes, stream>>>(a);
     PPF_CUDA(cudaGetLastError());
