@@ -18,9 +18,6 @@ namespace ppf {
 // 0..30; bin 30 is only reached at alpha == pi exactly).
 constexpr int kBins = 31;
 #define PPF_N_ANGLE_CELLS 31
-// Vote kernel launch shape: one 1024-thread block per SM.
-constexpr int kVoteThreads = 1024;
-constexpr int kVoteWarps = kVoteThreads / 32;
 // Most m_r rows of a chunk: m_r mod chunk takes the 11 bits above an entry's
 // 21-bit angle, and ppf_model_num_chunks reports the chunks.  (1659 rows of
 // 31 32-bit counters were what one block's shared memory held; at 64 bytes a
