@@ -88,28 +88,35 @@ __global__ void voxel_index_kernel(const float* __restrict__ xyz, size_t n, Grid
   }
 }
 
-// Mean of each voxel's points (stable order), written in voxel order.
+// Mean of each voxel's points (stable order), written in voxel order.  Eight
+// lanes per voxel, one per component (x y z of the point and the normal; two
+// idle): the sums run in point order, and the lanes of a voxel read a point's
+// 24 bytes together, four points ahead of the additions.  A thread per voxel
+// read them one component and one point at a time: 185 us for 10^6 points in
+// 68000 voxels.
 __global__ void centroid_kernel(const uint32_t* __restrict__ first, const uint32_t* __restrict__ count,
                                 size_t K, const uint32_t* __restrict__ order, const float* __restrict__ xyz,
                                 const float* __restrict__ nxyz, float* __restrict__ out_xyz,
                                 float* __restrict__ out_nxyz) {
-  for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < K; v += (size_t)gridDim.x * blockDim.x) {
-    float s[6] = {0, 0, 0, 0, 0, 0};
+  constexpr uint32_t kAhead = 4;
+  const uint32_t d = threadIdx.x & 7;
+  const float* const src = d < 3 ? xyz + d : nxyz + (d - 3);
+  float* const dst = d < 3 ? out_xyz + d : out_nxyz + (d - 3);
+  for (size_t v = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 3; v < K;
+       v += ((size_t)gridDim.x * blockDim.x) >> 3) {
     const uint32_t f = first[v], c = count[v];
-    for (uint32_t k = 0; k < c; ++k) {
-      const size_t p = order[f + k];
+    if (d >= 6) continue;
+    float s = 0.f;
+    uint32_t k = 0;
+    for (; k + kAhead <= c; k += kAhead) {
+      float x[kAhead];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        s[d] = __fadd_rn(s[d], xyz[3 * p + d]);
-        s[3 + d] = __fadd_rn(s[3 + d], nxyz[3 * p + d]);
-      }
-    }
-    const float cf = (float)c;
+      for (uint32_t j = 0; j < kAhead; ++j) x[j] = src[3 * (size_t)order[f + k + j]];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      out_xyz[3 * v + d] = __fdiv_rn(s[d], cf);
-      out_nxyz[3 * v + d] = __fdiv_rn(s[3 + d], cf);
+      for (uint32_t j = 0; j < kAhead; ++j) s = __fadd_rn(s, x[j]);
     }
+    for (; k < c; ++k) s = __fadd_rn(s, src[3 * (size_t)order[f + k]]);
+    dst[3 * v] = __fdiv_rn(s, (float)c);
   }
 }
 
@@ -201,7 +208,7 @@ size_t voxel_downsample(Context& ctx, const float* xyz_dev, const float* nxyz_de
   out_xyz.reserve(std::max<size_t>(K, 1) * 12);
   out_nxyz.reserve(std::max<size_t>(K, 1) * 12);
   if (K) {
-    centroid_kernel<<<grid_for(K, 128), 128, 0, st>>>(first.as<uint32_t>(), count.as<uint32_t>(), K,
+    centroid_kernel<<<grid_for(8 * K, 256, 16), 256, 0, st>>>(first.as<uint32_t>(), count.as<uint32_t>(), K,
                                                        order.as<uint32_t>(), xyz_dev, nxyz_dev,
                                                        out_xyz.as<float>(), out_nxyz.as<float>());
     PPF_CUDA(cudaGetLastError());
