@@ -31,6 +31,7 @@ constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kGreedyChunk = 1024;  // a thread and a row of bits per pose
 constexpr uint32_t kRowBits = kGreedyChunk / 32;
 constexpr uint32_t kSeedSlices = 32;     // shares of the existing clusters
+constexpr uint32_t kMatchLanes = 8;      // lanes per pose and share
 
 struct GPose {
   float4 a, b, c;  // R00 R01 R02 R10 | R11 R12 R20 R21 | R22 tx ty tz
@@ -122,32 +123,41 @@ __global__ void prep_kernel(const float* __restrict__ T, size_t U, GPose* __rest
   }
 }
 
-// blockIdx.y < kSeedSlices: the first cluster of a share of those existing
-// before the chunk [b, e) that each of its poses matches, the lowest over all
-// shares into assign.  Otherwise: 32 bits of each pose's row, bit j set if the
-// pose matches the chunk's earlier pose j.
+// kMatchLanes lanes per pose of the chunk [b, e).  blockIdx.y < kSeedSlices:
+// the first cluster that the pose matches in each lane's share of those
+// existing before the chunk, the lowest over all shares into assign.
+// Otherwise: 32 bits of each pose's row, bit j set if the pose matches the
+// chunk's earlier pose j.  A test is a long chain (square roots, atan2), so the
+// launch is as long as the tests that a lane makes in a row: with one lane per
+// pose and 32 tests each it took 43 us at 7 warps per SM, with 8 lanes 23 us
+// (4 and 16 lanes: the whole call 4% and 0.5% from that of 8).
 __global__ void __launch_bounds__(128) match_kernel(const GPose* __restrict__ poses, size_t b, size_t e,
                                                     const GPose* __restrict__ seeds,
                                                     const uint32_t* __restrict__ n_seeds,
                                                     uint32_t* __restrict__ assign, uint32_t* __restrict__ rows,
                                                     float tt, float rt) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b + i >= e) return;
-  const GPose p = poses[b + i];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kMatchLanes, part = t % kMatchLanes;
+  const bool in = b + i < e;
+  const GPose p = poses[in ? b + i : b];
   if (blockIdx.y < kSeedSlices) {
-    const uint32_t C = *n_seeds, share = (C + kSeedSlices - 1) / kSeedSlices;
-    const uint32_t end = min(C, (blockIdx.y + 1) * share);
-    for (uint32_t c = blockIdx.y * share; c < end; ++c)
+    if (!in) return;
+    const uint32_t C = *n_seeds, shares = kSeedSlices * kMatchLanes, share = (C + shares - 1) / shares;
+    const uint32_t begin = (blockIdx.y * kMatchLanes + part) * share, end = min(C, begin + share);
+    for (uint32_t c = begin; c < end; ++c)
       if (close_enough(p, seeds[c], tt, rt)) {
         atomicMin(assign + b + i, c);
         break;
       }
   } else {
-    const uint32_t w = blockIdx.y - kSeedSlices;
+    constexpr uint32_t kTests = 32 / kMatchLanes;
+    const uint32_t w = blockIdx.y - kSeedSlices, j0 = 32 * w + kTests * part;
     uint32_t bits = 0;
-    for (uint32_t j = 32 * w; j < min(i, 32 * w + 32); ++j)
-      if (close_enough(p, poses[b + j], tt, rt)) bits |= 1u << (j & 31);
-    rows[i * kRowBits + w] = bits;
+    if (in)
+      for (uint32_t j = j0; j < min(i, j0 + kTests); ++j)
+        if (close_enough(p, poses[b + j], tt, rt)) bits |= 1u << (j & 31);
+#pragma unroll
+    for (uint32_t o = 1; o < kMatchLanes; o <<= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+    if (in && part == 0) rows[i * kRowBits + w] = bits;
   }
 }
 
@@ -358,7 +368,7 @@ int cluster_poses_greedy_gpu(Context& ctx, const float* transforms_dev, const ui
   for (size_t b = 0; b < U; b += kGreedyChunk) {
     const size_t e = std::min(U, b + kGreedyChunk);
     const unsigned n = (unsigned)(e - b);
-    const dim3 grid((n + 127) / 128, kSeedSlices + (n + 31) / 32);
+    const dim3 grid((n * kMatchLanes + 127) / 128, kSeedSlices + (n + 31) / 32);
     match_kernel<<<grid, 128, 0, st>>>(P, b, e, seeds.as<GPose>(), seed_count, assign.as<uint32_t>(),
                                        rows.as<uint32_t>(), trans_thresh, rot_thresh);
     resolve_kernel<<<1, kGreedyChunk, kResolveSmem, st>>>(P, b, e, rows.as<uint32_t>(), seeds.as<GPose>(), seed_count,
