@@ -21,9 +21,10 @@ L2    : a 256 MB buffer is written on the engine's stream after every timed
 --profile-case: one lookup of the first model against the scene at
         ref_point_df=50 (same model tables, 10x fewer scene reference points),
         a short vote launch for ncu captures; prints the lookup's stats.
-roofline: the vote kernel (dominant), algorithmic bytes 4 B per vote
-        (one 32-bit run entry streamed per vote) + 32 B per scene pair
-        evaluated, over its CUDA-event time, against MEASURED_PEAKS.json.
+roofline: the vote kernel (dominant), algorithmic bytes 4 B per run entry
+        read (an entry is read once per group of scene pairs of one key) + 32 B
+        per scene pair evaluated, over its CUDA-event time, against
+        MEASURED_PEAKS.json.
 cpu_baseline: the CPU oracle (C++/OpenMP restatement of the reference path)
         on a bounded sample of scene reference points, scaled.
 served: (1 GPU) the small library preset of --serve on its first 24 requests:
@@ -56,18 +57,20 @@ METRIC = "registrations/s"
 TAU_D = (0.03, 0.035, 0.03, 0.05)
 REF_DF = 5
 THR = 0.3
-# DRAM bytes (read + write) per vote of the vote kernel for each of the
-# workload's four models, from ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum) on each model's profile case (--profile-all: the same
-# model tables against the scene at ref_point_df=50).  A model's entries are
-# re-read by concurrent work items while still in L2, so its DRAM bytes scale
-# with its votes; the 3047-point model's tables fit L2 entirely.
-DRAM_BYTES_PER_VOTE = (0.04995, 0.03125, 0.04418, 0.001337)
-# Shared-memory bank wavefronts per warp-wide atomic of the vote kernel, from
-# ncu on the first model's profile case
-# (l1tex__data_pipe_lsu_wavefronts_mem_shared_op_atom.sum over
-# smsp__inst_executed_op_shared_atom.sum).
-VOTE_WAVEFRONTS_PER_ATOMIC = 1.94
+# Of the vote kernel, for each of the workload's four models, per vote on the
+# model's profile case (--profile-all: the same model tables against the scene
+# at ref_point_df=50).  DRAM bytes (dram__bytes_read.sum +
+# dram__bytes_write.sum); a model's entries are re-read by concurrent work items
+# while still in L2, so they scale with its votes.  Warp-wide shared atomics
+# (smsp__inst_executed_op_shared_atom.sum).  Run entries read, one per entry and
+# group of scene pairs (counted by an instrumented copy of the kernel).
+DRAM_BYTES_PER_VOTE = (0.03263, 0.05414, 0.09187, 0.002565)
+WARP_ATOMICS_PER_VOTE = (0.013503, 0.018633, 0.023931, 0.005789)
+ENTRIES_PER_VOTE = (0.0348, 0.0609, 0.0922, 0.01296)
+# Shared-memory bank wavefronts per warp-wide atomic of the vote kernel
+# (l1tex__data_pipe_lsu_wavefronts_mem_shared_op_atom.sum over the atomics:
+# 2.71, 2.87, 3.24 and 2.81, weighted by the workload's atomics).
+VOTE_WAVEFRONTS_PER_ATOMIC = 2.85
 
 
 def shared_atomic_peaks(device):
@@ -100,11 +103,9 @@ def shared_atomic_peaks(device):
 
 def atomic_roofline(peaks, votes, vote_s, sm_mhz, n_sm):
     """The vote kernel's warp-wide shared atomics per SM-cycle against the
-    probe's rate.  Every vote is one lane of a warp-wide atomic; the unrolled
-    passes keep all 32 lanes busy and the masked remainder of a segment holds
-    about 1% of the votes, so the kernel issues about votes / 32 of them.  The
-    ceiling at the kernel's own conflict level interpolates the probe's cycles
-    per atomic linearly between one and two wavefronts."""
+    probe's rate, for `votes` lanes of full warp-wide atomics (32 per atomic).
+    The ceiling at the kernel's own conflict level extends the probe's cycles
+    per atomic at one and two wavefronts linearly."""
     if not peaks or vote_s <= 0 or not sm_mhz:
         return None
     achieved = votes / 32.0 / (vote_s * sm_mhz * 1e6 * n_sm)
@@ -402,7 +403,7 @@ def run_serve(args):
             out.append(np.asarray(p[0]))
         return out
 
-    # warm-up (pool, tuner, candidate hints): every request for the small
+    # warm-up (pool, candidate hints): every request for the small
     # preset, the first one for the library configs
     plain_all(None if args.serve_preset == "small" else reqs[:1])
     ctx.synchronize()
@@ -649,7 +650,7 @@ def main():
     launches0 = ctx.kernel_launches
     vote_ms = 0.0
     votes = 0
-    traffic = 0.0
+    traffic = entries = atomics = 0.0
     pairs = 0
     with ClockSampler(local, args.clock_interval_ms, args.clocks_dir) as clk:
         ev0 = torch.cuda.Event(enable_timing=True)
@@ -662,6 +663,8 @@ def main():
                 vote_ms += s["vote_ms"]
                 votes += s["n_votes"]
                 traffic += s["n_votes"] * DRAM_BYTES_PER_VOTE[k]
+                entries += s["n_votes"] * ENTRIES_PER_VOTE[k]
+                atomics += s["n_votes"] * WARP_ATOMICS_PER_VOTE[k]
         ev1.record(stream)
         ev1.synchronize()
         if dist:
@@ -676,8 +679,8 @@ def main():
         sys.exit(3)
     n_ref = (len(spec.scene) + REF_DF - 1) // REF_DF
     # every (scene reference point, chunk) work item walks the whole scene, so
-    # a model of C chunks evaluates each scene pair C times
-    pairs = n_ref * len(spec.scene) * sum(chunks) * args.steps
+    # a scene reference point's pairs are evaluated once for all chunks of a model
+    pairs = n_ref * len(spec.scene) * len(chunks) * args.steps
     ms_max = reduce_max(dist, ms, dev)
     regs = world * len(spec.models) * args.steps
     value = regs / (ms_max / 1000.0)
@@ -716,9 +719,9 @@ def main():
         return
     peak, peak_kind = measured_peaks()
     clocks = clk.summary()
-    atomics = atomic_roofline(shared_atomic_peaks(local), votes, vote_ms / 1000.0, clocks.get("sm_mhz"),
-                              torch.cuda.get_device_properties(dev).multi_processor_count)
-    alg_bytes = 4.0 * votes + 32.0 * pairs
+    shared = atomic_roofline(shared_atomic_peaks(local), 32.0 * atomics, vote_ms / 1000.0, clocks.get("sm_mhz"),
+                             torch.cuda.get_device_properties(dev).multi_processor_count)
+    alg_bytes = 4.0 * entries + 32.0 * pairs
     vote_s = vote_ms / 1000.0
     achieved = alg_bytes / vote_s / 1e9 if vote_s > 0 else 0.0
     line = {
@@ -746,17 +749,16 @@ def main():
                      "kernel": "vote_batch_kernel (one launch per step: the four lookups' vote passes)",
                      "traffic": traffic / args.steps,
                      "traffic_note": "DRAM bytes per launch: measured bytes per vote of each model's profile "
-                                     "case times its votes; the entries are served from L2 (about 0.5% of the "
-                                     "algorithmic bytes reach DRAM); the kernel is latency-bound on its L2 entry "
-                                     "loads, with the l1tex data pipe (shared atomics + loads) at 69% of peak on the "
-                                     "profile case",
+                                     "case times its votes; the entries are served from L2; the kernel is bound "
+                                     "by the l1tex data pipe (shared-memory wavefronts, 79-81% of peak on the "
+                                     "profile cases of the models with most votes, 57-61% on the others)",
                      "alg_bytes_per_launch": alg_bytes / args.steps,
-                     "alg_bytes_rule": "4 B per vote + 32 B per scene pair evaluated (pairs x vote chunks of the model)",
+                     "alg_bytes_rule": "4 B per run entry and group of scene pairs + 32 B per scene pair evaluated",
                      "vote_chunks": chunks,
                      "vote_ms_per_launch": vote_ms / args.steps,
-                     "shared_atomics": atomics},
+                     "shared_atomics": shared},
         "gpu_launches": int(launches),
-        "vote_segments_tuned": [int(s["vote_segment"]) for s in stats[0]],
+        "vote_segments": [int(s["vote_segment"]) for s in stats[0]],
         "recall": recall,
         "clocks": clocks,
     }

@@ -3,11 +3,11 @@
 // scene pair features or individual votes.
 //
 // One work item = (scene reference point s_r, a range of chunks of model
-// reference points).  A persistent block (1024 threads, one per SM) takes
-// items from an atomic counter.  For its s_r it
-//  1. walks the scene points in tiles of 1024: one pair feature, FNV key and
-//     run lookup per thread; matched pairs ("events") go to a list in shared
-//     memory and are counted per model run in a small hash table,
+// reference points).  A persistent block (1024 threads, one per SM, or two of
+// 512 for small models) takes items from an atomic counter.  For its s_r it
+//  1. walks the scene points, two per lane: one pair feature and run lookup
+//     each; matched pairs ("events") go to a list in shared memory and are
+//     counted per model run in a small hash table,
 //  2. groups the list by run (counting sort) and cuts each group into pieces
 //     of at most kPieceEvents events,
 //  3. per chunk, lets warps take units (a piece x a segment of the run's
@@ -23,8 +23,8 @@
 // pair reads and counts every entry G times.  A piece of G events adds a
 // whole 30-bin histogram per entry instead (sweep_unit).  Vote pass at
 // ref_point_df 50, a shared atomic per vote against this: 47.1 / 17.7 / 19.5 /
-// 72.8 ms against 23.0 / 12.8 / 13.9 / 19.2 ms for the bench's four models,
-// and 6.7 against 5.9 ms for the 2000-point model and 10000-point scene.  What
+// 72.8 ms against 20.6 / 10.9 / 12.1 / 15.9 ms for the bench's four models,
+// and 6.4 against 5.3 ms for the 2000-point model and 10000-point scene.  What
 // bounds it now: shared-memory wavefronts of the swept entries (about 53 per
 // 32 entries, two thirds of the time at long sub-runs) and issue slots of the
 // events between them (short sub-runs).
