@@ -609,6 +609,10 @@ __global__ void __launch_bounds__(kWarpBlock, 8) cluster_warp_kernel(GroupArgs a
   const uint32_t lanes_below = (1u << lane) - 1u;
   float c = 1;
   float3 to = t;
+  // The marked sources' tests, kUnroll reads of the list in flight (the sums
+  // keep their order).  After the votes of 5.6 M poses, 2 / 4 / 8 / 16 at a time:
+  // 10.43 / 10.21 / 10.04 / 10.64 ms; averaged 13.37 / 13.30 / 13.60 / -.
+  constexpr int kUnroll = AVG ? 4 : 8;
   for (uint32_t used = 0; used < issued; ++used) {
     produce();
     cp_async_wait<kRingStages - 1>();
@@ -635,7 +639,7 @@ __global__ void __launch_bounds__(kWarpBlock, 8) cluster_warp_kernel(GroupArgs a
       }
       __syncwarp();
       const int n = __popc(mask);
-#pragma unroll 2
+#pragma unroll kUnroll
       for (int e = 0; e < n; ++e) {
         const float4 sv = mk[0][e], wv = mk[1][e];
         if (cluster_match_t<TT>(a, q, t, sv, wv, rot_sq8)) {
