@@ -581,7 +581,12 @@ __device__ __forceinline__ bool walk_scene(const VoteArgs& a, uint32_t sr, bool 
     __syncwarp();
     const uint32_t n = min(ws.n_near, 32u);
     if (n == 0) break;
-    if (*(volatile uint32_t*)&sh.n_gr > kGroupLimit) {
+    // One lane reads the count for its warp: other warps raise it meanwhile, and
+    // lanes that read it for themselves could part here and leave the others
+    // in the ballots below.
+    uint32_t groups = 0;
+    if (lane == 0) groups = *(volatile uint32_t*)&sh.n_gr;
+    if (__shfl_sync(0xffffffffu, groups, 0) > kGroupLimit) {
       full = true;
       break;
     }
