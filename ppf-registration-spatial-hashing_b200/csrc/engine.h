@@ -14,10 +14,6 @@ struct ppf_context_s;
 
 namespace ppf {
 
-// Angle bins per model reference point in the vote accumulator (alpha bins
-// 0..30; bin 30 is only reached at alpha == pi exactly).
-constexpr int kBins = 31;
-#define PPF_N_ANGLE_CELLS 31
 // Most m_r rows of a chunk: m_r mod chunk takes the 11 bits above an entry's
 // 21-bit angle, and ppf_model_num_chunks reports the chunks.  (1659 rows of
 // 31 32-bit counters were what one block's shared memory held; at 64 bytes a
@@ -127,7 +123,6 @@ struct LookupState {
   DevBuf trans;       // float U*3 (after clustering)
   DevBuf trans0;      // float U*3 (before clustering)
   DevBuf quats;       // float U*4
-  DevBuf cell_keys;   // uint32 U
   DevBuf scores;      // float U
   DevBuf cells_sorted, cells_map, cells_uniq, cells_first, cells_count;
   DevBuf cells3;      // int4 U: integer cell of each pose

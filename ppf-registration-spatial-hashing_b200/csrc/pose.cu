@@ -142,8 +142,7 @@ struct PoseArgs {
   float* trans0;
   float* quats;
   float* weighted;
-  uint32_t* cell_keys;
-  uint32_t* cells_sorted;  // cell_keys again, to be sorted
+  uint32_t* cells_sorted;  // cell keys, sorted in place by the clustering
   int4* cells3;
 };
 
@@ -182,9 +181,7 @@ __global__ void poses_kernel(PoseArgs a) {
     a.quats[4 * i + 3] = q.w;
     a.weighted[i] = a.m_w[mr] * a.counts[i];
     int3 c = trans_cell(t, a.d_dist);
-    const uint32_t key = cell_key(c.x, c.y, c.z);
-    a.cell_keys[i] = key;
-    a.cells_sorted[i] = key;
+    a.cells_sorted[i] = cell_key(c.x, c.y, c.z);
     a.cells3[i] = make_int4(c.x, c.y, c.z, 0);
   }
 }
@@ -923,7 +920,6 @@ void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState
   a.trans0 = grow<float>(st.trans0, U * 3);
   a.quats = grow<float>(st.quats, U * 4);
   a.weighted = grow<float>(st.weighted, U);
-  a.cell_keys = grow<uint32_t>(st.cell_keys, U);
   a.cells_sorted = grow<uint32_t>(st.cells_sorted, U);
   a.cells3 = grow<int4>(st.cells3, U);
   grow<float>(st.trans, U * 3);
@@ -937,7 +933,6 @@ void compute_poses(Context& ctx, const Model& m, const SceneData& s, LookupState
     PPF_CUDA(cudaMemsetAsync(st.trans.ptr, 0, U * 12, stream));
     PPF_CUDA(cudaMemsetAsync(a.quats, 0, U * 16, stream));
     PPF_CUDA(cudaMemsetAsync(a.weighted, 0, U * 4, stream));
-    PPF_CUDA(cudaMemsetAsync(a.cell_keys, 0, U * 4, stream));
     PPF_CUDA(cudaMemsetAsync(st.scores.ptr, 0, U * 4, stream));
     return;
   }
