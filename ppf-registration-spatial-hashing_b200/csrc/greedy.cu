@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(1024) top3_average_kernel(const GPose* __restr
     const bool mem = i < U && assign[i] == c;
     const uint32_t bal = __ballot_sync(0xffffffffu, mem);
     if (lane == 0) s_off[warp] = __popc(bal);
+    __syncwarp();  // the warp reaches the barrier converged, as in block_sync
     const uint32_t cnt = (uint32_t)__syncthreads_count(mem);
     if (cnt == 0) continue;
     if (mem) {

@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(256) lut_kernel(const uint32_t* __restrict__ h
     if (nd < kLutRows) lut[nd * kAngleCombos + c] = run;
     any = any || run != 0xffffffffu;
   }
+  __syncwarp();  // the lanes leave the loop at different times
   if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(row_flags + nd / 32, 1u << (nd % 32));
 }
 

@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kThreads, 2) rs_onesweep(
     }
     s_global[tid] = pass_base + excl - start;
   }
+  __syncwarp();  // the lanes leave the look-back at different times
   __syncthreads();
   const uint32_t last = (uint32_t)(n - 1);
   for (uint32_t p = tid; p < valid; p += kThreads) {
