@@ -188,7 +188,7 @@ std::vector<LookupOut> lookup_batch(Context& ctx, const std::vector<Model*>& mod
       auto it = ctx.cand_hints.find(model_signature(*models[i]));
       if (it != ctx.cand_hints.end()) hint = it->second;
     }
-    reqs[i].cap = hint ? hint + hint / 4 + 65536 : (size_t(1) << 22);
+    reqs[i].cap = batch_cells(hint);
     want += reqs[i].cap;
   }
   if (want > kBudgetCells)

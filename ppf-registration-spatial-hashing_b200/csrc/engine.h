@@ -244,6 +244,9 @@ struct LookupOut {
   size_t cand_hint = 0;  // candidate cells to provide for the next pass of this model
 };
 void init_context(Context& c, int device, bool kept = true);
+// Candidate cells that a batch provides for a request whose model's last pass
+// had `hint` of them (0: no pass yet).
+inline size_t batch_cells(size_t hint) { return hint ? hint + hint / 4 + 65536 : size_t(1) << 22; }
 // Lookups of (models[i], scenes[i]) with one batched vote pass.  states:
 // per-request lookup state (nullptr: each model's own `last`); caps:
 // per-request candidate capacity hints (nullptr: the models' last passes).

@@ -51,6 +51,7 @@ struct Server {
   int device = 0;
   std::vector<Model*> models;        // borrowed library
   std::vector<size_t> hints;         // candidate cells of each model's last pass
+  std::vector<size_t> kept;          // kept votes of each model's last pass
   size_t budget = 0, in_use = 0;
   uint32_t max_batch = 16;
   std::vector<std::unique_ptr<ppf_context_s>> ctxs;
@@ -63,15 +64,16 @@ struct Server {
   bool stop = false;
 
   // Device bytes a request holds while in flight, per target model: the
-  // scene as float4 points and normals, and for the expected candidate count
-  // c its candidate cells (12 B each, with 25% headroom) and its lookup state
-  // (kept votes, about c / 2, at ~230 B each).
+  // scene as float4 points and normals, its candidate cells (12 B each, and
+  // 12 B each again while they are ordered) and its kept votes (196 B of
+  // lookup state each, 20 B of sort scratch).  Both counts are those of the
+  // model's last pass, since their ratio runs from 1 to 60 between scenes;
+  // before the first pass half a million kept votes are assumed.  A worker's
+  // context holds about 30 MB besides, whatever runs on it.
   size_t need_bytes(const Request& r) const {
     size_t b = 0;
-    for (uint32_t j : r.targets) {
-      const size_t c = std::max<size_t>(hints[j], size_t(1) << 20);
-      b += 32 * r.n + 15 * c + 115 * c;
-    }
+    for (uint32_t j : r.targets)
+      b += 32 * r.n + 24 * batch_cells(hints[j]) + 216 * (hints[j] ? kept[j] : size_t(1) << 19);
     return b;
   }
 
@@ -110,6 +112,7 @@ struct Server {
         r->stats[t] = out[k].stats;
         if (out[k].status != PPF_OK) r->status = out[k].status;
         hints[r->targets[t]] = out[k].cand_hint;
+        kept[r->targets[t]] = out[k].stats.n_kept;
       }
     }
   }
@@ -174,9 +177,11 @@ Server* server_create(int device, const std::vector<Model*>& models, size_t memo
   std::unique_ptr<Server> s(new Server());
   s->models = models;
   s->hints.resize(models.size());
+  s->kept.resize(models.size());
   for (size_t j = 0; j < models.size(); ++j) {
     PPF_REQUIRE(models[j], PPF_ERR_INVALID_ARGUMENT, "null model in the library");
     s->hints[j] = models[j]->cand_hint;
+    s->kept[j] = models[j]->last.U;
   }
   // the library's tables may still be in flight on their own contexts' streams
   PPF_CUDA(cudaDeviceSynchronize());
