@@ -678,8 +678,9 @@ def main():
         sys.stderr.write(f"bench: poses of models {changed} changed between warm-up and timed steps\n")
         sys.exit(3)
     n_ref = (len(spec.scene) + REF_DF - 1) // REF_DF
-    # every (scene reference point, chunk) work item walks the whole scene, so
-    # a scene reference point's pairs are evaluated once for all chunks of a model
+    # each scene pair once per model, the fewest it takes: chunks shared out
+    # over several work items, and scenes whose pairs do not fit a list, are
+    # walked again
     pairs = n_ref * len(spec.scene) * len(chunks) * args.steps
     ms_max = reduce_max(dist, ms, dev)
     regs = world * len(spec.models) * args.steps
@@ -753,7 +754,7 @@ def main():
                                      "by the l1tex data pipe (shared-memory wavefronts, 79-81% of peak on the "
                                      "profile cases of the models with most votes, 57-61% on the others)",
                      "alg_bytes_per_launch": alg_bytes / args.steps,
-                     "alg_bytes_rule": "4 B per run entry and group of scene pairs + 32 B per scene pair evaluated",
+                     "alg_bytes_rule": "4 B per run entry and group of scene pairs + 32 B per scene pair and model",
                      "vote_chunks": chunks,
                      "vote_ms_per_launch": vote_ms / args.steps,
                      "shared_atomics": shared},

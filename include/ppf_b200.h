@@ -183,7 +183,9 @@ ppf_status ppf_voxel_downsample(ppf_context_t ctx, const float* xyz, const float
  * memory_budget bytes; up to max_batch admitted requests share one batched
  * vote pass.  Workers run concurrently, so requests that arrive while others
  * are on the GPU are admitted as memory frees and overlap them.  A request
- * larger than the whole budget runs alone. */
+ * larger than the whole budget runs alone.  The estimate takes the candidate
+ * cells and kept votes of the target model's last lookup; the workers' contexts
+ * hold about 30 MB each besides. */
 ppf_status ppf_server_create(int device, uint64_t n_models, const ppf_model_t* models,
                              uint64_t memory_budget, uint32_t n_workers, uint32_t max_batch,
                              ppf_server_t* out);

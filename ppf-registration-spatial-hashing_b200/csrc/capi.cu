@@ -618,9 +618,10 @@ ppf_status ppf_registration(ppf_context_t ctx, uint64_t n_scenes, const float* c
     using ModelPtr = std::unique_ptr<ppf_model_s, ppf_status (*)(ppf_model_t)>;
     using ScenePtr = std::unique_ptr<ppf_scene_s, ppf_status (*)(ppf_scene_t)>;
     // The reference builds each model again for every scene; a model built
-    // once gives the same results.  Models are built in groups whose tables
-    // (about 17 bytes per ordered pair) fit a device budget, and all (scene,
-    // model) pairs of a group share one batched vote pass.
+    // once gives the same results.  Models are built in groups whose tables fit
+    // a device budget (12 bytes per ordered pair stay; 17 are charged, for the
+    // build in progress), and all (scene, model) pairs of a group share one
+    // batched vote pass.
     constexpr double kGroupBytes = 48e9;
     for (uint64_t j0 = 0; j0 < n_models;) {
       uint64_t j1 = j0;

@@ -27,10 +27,10 @@ constexpr uint32_t kFlagRows = 1024;
 // Angle quantum on the host (include/kernel.h:16 evaluated in float).
 #define PPF_D_ANGLE_HOST ((2.0f * 3.141592654f) / float(30))
 
+constexpr size_t kHostBytes = 4096;  // of Context::host
+
 // Every DevBuf member must be released in ~Context (capi.cu) before the
 // stream its blocks are freed on is destroyed.
-constexpr size_t kHostBytes = 4096;
-
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -168,12 +168,13 @@ struct VoteResult {
   uint64_t n_needed = 0;  // cells the first launch's items asked for (sizes the next buffer)
   float vote_ms = 0;
 };
-// Runs the vote pass.  emit_all: emit every nonzero cell (no threshold);
-// floor >= 0 forces the emission floor.  Candidates land in
-// ctx.cand_codes / ctx.cand_counts.
+// Shared-memory sizes of the vote kernels, the same for every launch.
 void init_vote_kernels(int smem_limit);
 // The vote blocks' 32-bit counters (ctx.vote_spill).
 void reserve_vote_spill(Context& ctx);
+// Runs the vote pass.  emit_all: emit every nonzero cell (no threshold);
+// floor >= 0 forces the emission floor.  Candidates land in
+// ctx.cand_codes / ctx.cand_counts.
 VoteResult run_votes(Context& ctx, const Model& m, const SceneData& s, bool emit_all, float floor);
 // One request of a batched vote pass: its candidate cells land in its own
 // buffers (cap cells, grown if they do not fit).

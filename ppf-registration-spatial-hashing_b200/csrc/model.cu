@@ -676,9 +676,9 @@ void build_model(Context& ctx, ModelTables& t, const float* xyz, const float* nx
               "model tables inconsistent: check " + std::to_string(badh[0]) + " at " +
                   std::to_string(badh[1]));
   if (!ctx.checks) t.keys.release();  // only the build's sorts used the runs in map order
-  // The sorts keep scratch of about 16 bytes per sorted pair for reuse by
-  // later builds; past 2^28 pairs (16k-point models) that is gigabytes, so
-  // it goes back to the pool now.
+  // The sorts keep scratch of 8 bytes per sorted pair (21 where the vote
+  // order's words need 64 bits) for reuse by later builds; past 2^28 pairs
+  // (16k-point models) that is gigabytes, so it goes back to the pool now.
   if (t.P > (size_t(1) << 28)) {
     ctx.sort32.release();
     ctx.sort64.release();

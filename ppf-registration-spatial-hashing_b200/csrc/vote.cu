@@ -233,11 +233,16 @@ constexpr int kBlocksPerSm = 2;
 
 // The narrow shape where the chunks of all requests fit it, there are more
 // items than SMs (an item alone on an SM is done sooner by a wide block) and no
-// scene is so large that its events would often need a second list.  Wide to
-// narrow, vote pass in us: model 300 in 1000 points, every one a reference
-// point, 208 to 144; 200 in 5000 / 3 432 to 269; 700 in 4500 / 5 281 to 260;
-// 831 in 6000 / 5 645 to 558; 300 in 20000 / 9 1484 to 1096; past the bound 700
-// in 60000 / 51 2515 to 2402, but 3715 to 4051 for a flat model.
+// scene is so large that its events would often need a second list.  Time of
+// the vote pass in wide blocks over narrow ones, models in scenes of 3 to 8
+// times their points, two quanta:
+//   model points                    100        300        511        700        831
+//   superellipsoid, torus, capsules 1.30-1.63  1.26-1.48  1.18-1.37  1.11-1.31  1.07-1.28
+//   spheres on a slab               1.31-1.38  1.16-1.25  1.00-1.14  0.96-1.08  0.87-1.07
+// The flat model's lists outgrow a narrow block from about 700 points in 5600
+// on; its longer groups gain most from the grouping itself.  Past the scene
+// bound 700 in 60000 / 51 takes 2515 us wide and 2402 narrow, a flat model 3715
+// and 4051.
 constexpr uint32_t kNarrowScene = 8 * narrow::kEvents;
 bool narrow_blocks(uint32_t rows, uint32_t scene, size_t items) {
   return rows <= kNarrowRows && scene <= kNarrowScene && items > (size_t)sm_count();

@@ -874,7 +874,7 @@ __device__ __forceinline__ void vote_units(const VoteArgs& a, VoteShared& sh, Vo
   while (u < u1) {
     // piece p with pc_unit[p] <= u < pc_unit[p + 1] (pc_unit is
     // nondecreasing): one ballot over every stride-th piece, then over the
-    // stride (at most 49) pieces behind it
+    // stride (at most (kMaxPieces + 31) / 32, 53 in a wide block) pieces behind it
     const uint32_t blk =
         31u - __clz(__ballot_sync(0xffffffffu, lane * stride <= n_pieces && pc_unit[min(lane * stride, n_pieces)] <= u));
     uint32_t p = blk * stride;
